@@ -245,6 +245,44 @@ int setup_staged(lbm_t *h, int want_stages)
     return LBM_OK;
 }
 
+// Vector width and launch count of an iteration of the direct and narrow
+// variants: h->step_vb > 0, step_kernel with vectors of so many bytes, one
+// launch; 0, pull_kernel's two launches with 16-byte vectors (16-bit storage).
+//
+// Wide vectors cost registers and give few threads: a small lattice wants
+// one or two sites per thread (its time is the latency of one thread's work
+// after a launch), a large one the fewest instructions.  us per iteration in
+// replayed graphs, 4- / 8- / 16-byte vectors, one launch; two launches:
+//   FP16  32^3  2.3 / 2.8 / 4.1; 4.9   64^3 5.8 / 5.1 / 6.7; 6.0
+//         96^3 14.1 / 11.9 / 11.8; 12.4   128^3 34.2 / 31.3 / 29.1; 30.0
+//         200^3  122 / 111 / 104.7; 103.5   256^3  253 / 211 / 208; 203
+//         512^3 1897 / 1648 / 1610; 1527
+//   BF16  32^3  2.3 / 2.6 / 3.6; 6.0   64^3 5.6 / 5.0 / 6.5; 7.0
+//         128^3 31.6 / 29.1 / 28.6; 31.4   200^3 105.5; 106.3   256^3 208; 205
+//   FP32  32^3  2.9 / 3.2 / 4.9; 3.8   64^3 8.1 / 7.5 / 9.0; 7.9
+//         128^3 57 / 48.0 / 55; 50.7   256^3 400 / 360 / 415; 375
+//         512^3 3157 / 2910 / 3217; 2950
+//   FP64 (8- / 16-byte) 16^3 13.3 / 20.9; 24   32^3 19.6 / 23.9; 24
+//         128^3 989 / 1050; 1045   256^3 7767 / 8014; 7987
+int step_shape(int kernel, int prec, int dim)
+{
+    const bool s16 = prec == LBM_FP16 || prec == LBM_BF16;
+    if (kernel == LBM_KERNEL_NARROW) return 8;
+    if (kernel == LBM_KERNEL_DIRECT && !s16) return 16;
+    if (prec == LBM_FP64) return 8;
+    if (prec == LBM_FP32) return dim <= 40 ? 4 : 8;
+    if (dim > 192) return 0;
+    if (kernel == LBM_KERNEL_DIRECT) return 16;
+    return dim <= 40 ? 4 : dim <= 72 ? 8 : 16;
+}
+
+// The two launches of an iteration with 16-byte vectors, face rows on sf.
+cudaError_t launch_rows(const lbm_t *h, int mode, const lbm::StepArgs &a, cudaStream_t sf)
+{
+    return h->prec == LBM_FP16 ? lbm::launch_rows_f16(mode, a, h->step_block, h->stream, sf)
+                               : lbm::launch_rows_bf16(mode, a, h->step_block, h->stream, sf);
+}
+
 cudaError_t launch_pull(const lbm_t *h, int mode, const lbm::StepArgs &a, unsigned *nparts = nullptr)
 {
     if (h->kernel == LBM_KERNEL_AA) {
@@ -255,6 +293,14 @@ cudaError_t launch_pull(const lbm_t *h, int mode, const lbm::StepArgs &a, unsign
         default: return lbm::launch_aa_bf16(mode, a, h->block, h->stream, nparts);
         }
     }
+    if (mode == lbm::MODE_REDUCE) {
+        switch (h->prec) {
+        case LBM_FP32: return lbm::launch_reduce_f32(a, h->block, h->stream, nparts);
+        case LBM_FP64: return lbm::launch_reduce_f64(a, h->block, h->stream, nparts);
+        case LBM_FP16: return lbm::launch_reduce_f16(a, h->block, h->stream, nparts);
+        default: return lbm::launch_reduce_bf16(a, h->block, h->stream, nparts);
+        }
+    }
     if (h->kernel == LBM_KERNEL_STAGED && (mode == lbm::MODE_STEP || mode == lbm::MODE_STEP_MACRO)) {
         switch (h->prec) {
         case LBM_FP32: return lbm::launch_staged_f32(mode, a, h->sgrid, h->sblock, h->ssmem, h->stream);
@@ -263,18 +309,12 @@ cudaError_t launch_pull(const lbm_t *h, int mode, const lbm::StepArgs &a, unsign
         default: return lbm::launch_staged_bf16(mode, a, h->sgrid, h->sblock, h->ssmem, h->stream);
         }
     }
-    if (h->kernel == LBM_KERNEL_NARROW && mode != lbm::MODE_REDUCE) {
-        switch (h->prec) {
-        case LBM_FP32: return lbm::launch_narrow_f32(mode, a, h->block, h->stream);
-        case LBM_FP16: return lbm::launch_narrow_f16(mode, a, h->block, h->stream);
-        default: return lbm::launch_narrow_bf16(mode, a, h->block, h->stream);
-        }
-    }
+    if (!h->step_vb) return launch_rows(h, mode, a, h->stream);
     switch (h->prec) {
-    case LBM_FP32: return lbm::launch_pull_f32(mode, a, h->block, h->stream, nparts);
-    case LBM_FP64: return lbm::launch_pull_f64(mode, a, h->block, h->stream, nparts);
-    case LBM_FP16: return lbm::launch_pull_f16(mode, a, h->block, h->stream, nparts);
-    default: return lbm::launch_pull_bf16(mode, a, h->block, h->stream, nparts);
+    case LBM_FP32: return lbm::launch_step_f32(h->step_vb, mode, a, h->step_block, h->stream);
+    case LBM_FP64: return lbm::launch_step_f64(h->step_vb, mode, a, h->step_block, h->stream);
+    case LBM_FP16: return lbm::launch_step_f16(h->step_vb, mode, a, h->step_block, h->stream);
+    default: return lbm::launch_step_bf16(h->step_vb, mode, a, h->step_block, h->stream);
     }
 }
 
@@ -288,25 +328,20 @@ bool macro_within(int64_t it0, int G, int macro_every)
     return next <= it0 + G;
 }
 
-bool splits(const lbm_t *h) { return h->kernel == LBM_KERNEL_DIRECT || h->kernel == LBM_KERNEL_NARROW; }
+// the two-launch iterations
+bool splits(const lbm_t *h) { return h->kernel != LBM_KERNEL_AA && h->kernel != LBM_KERNEL_STAGED && !h->step_vb; }
 
-// One iteration (MODE_STEP or MODE_STEP_ADJ) of the direct / narrow variants
-// with its face-row launch on the side stream, forked from and joined back
-// into the handle's stream, so that (in a captured graph: as a second
-// branch) it runs beside the interior-row launch; the two write disjoint rows
-// of the output and read the same input.
+// One two-launch iteration (MODE_STEP or MODE_STEP_ADJ) with its face-row
+// launch on the side stream, forked from and joined back into the handle's
+// stream, so that (in a captured graph: as a second branch) it runs beside the
+// interior-row launch; the two write disjoint rows of the output and read the
+// same input.
 cudaError_t split_iteration(const lbm_t *h, int mode, const lbm::StepArgs &a)
 {
     cudaError_t e = cudaEventRecord(h->ev_fork, h->stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->ev_fork, 0);
     if (e != cudaSuccess) return e;
-    const int vb = h->kernel == LBM_KERNEL_NARROW ? 8 : 16;
-    switch (h->prec) {
-    case LBM_FP32: e = lbm::launch_split_f32(vb, mode, a, h->block, h->stream, h->side); break;
-    case LBM_FP64: e = lbm::launch_split_f64(vb, mode, a, h->block, h->stream, h->side); break;
-    case LBM_FP16: e = lbm::launch_split_f16(vb, mode, a, h->block, h->stream, h->side); break;
-    default: e = lbm::launch_split_bf16(vb, mode, a, h->block, h->stream, h->side); break;
-    }
+    e = launch_rows(h, mode, a, h->side);
     // join even after a failed launch, so the capture can end
     const cudaError_t ej = cudaEventRecord(h->ev_join, h->side);
     const cudaError_t ew = ej == cudaSuccess ? cudaStreamWaitEvent(h->stream, h->ev_join, 0) : ej;
@@ -316,8 +351,8 @@ cudaError_t split_iteration(const lbm_t *h, int mode, const lbm::StepArgs &a)
 // Replay (capturing on first use) the graph of h->graph_iters plain
 // iterations that starts from buffer h->cur.  The kernels' arguments are
 // fixed per parity (the two buffers ping-pong), so two graphs cover every
-// call.  With the direct / narrow kernels each iteration's face-row launch is
-// a branch beside its interior-row launch.
+// call.  In two-launch iterations the face-row launch is a branch beside the
+// interior-row launch.
 cudaError_t replay_graph(lbm_t *h)
 {
     cudaGraphExec_t &exec = h->graph_exec[parity(h)];
@@ -565,14 +600,14 @@ int lbm_init(lbm_t **out, const lbm_config *c)
         // the copy source (lidh) must outlive the copy
         LBM_CUDA(cudaStreamSynchronize(h->stream));
 
-        // iteration kernel: the fastest variant measured at 512^3 on GB300 --
-        // 16-byte vectors for 16-bit storage and FP64, 8-byte vectors for FP32
-        int want = c->kernel;
-        if (want == LBM_KERNEL_AUTO) want = prec == LBM_FP32 ? LBM_KERNEL_NARROW : LBM_KERNEL_DIRECT;
+        const int want = c->kernel;
         h->kernel = aa ? LBM_KERNEL_AA : LBM_KERNEL_DIRECT;
-        if (want == LBM_KERNEL_NARROW && prec != LBM_FP64) {
-            h->kernel = LBM_KERNEL_NARROW;
-        }
+        if (want == LBM_KERNEL_NARROW && prec != LBM_FP64) h->kernel = LBM_KERNEL_NARROW;
+        h->step_vb = step_shape(want == LBM_KERNEL_NARROW && prec == LBM_FP64 ? LBM_KERNEL_AUTO : want, prec, dim);
+        // 64-thread blocks: a finer last wave (FP16 512^3, us per iteration:
+        // 32 threads 1539, 64 1527, 96 1556, 128 1558; FP32 200^3: 64 174.6,
+        // 128 175.9, 256 183)
+        h->step_block = c->block_threads > 0 ? block : 64u;
         if (want == LBM_KERNEL_STAGED) {
             const int r = setup_staged(h, c->stages);
             if (r == LBM_OK) h->kernel = LBM_KERNEL_STAGED;

@@ -339,6 +339,25 @@ __device__ __forceinline__ float deq_scaled(int i, float drho, float rho, float 
 // StepArgs::u: u_x, u_y, u_z of FLUID sites; rho, 0, 0 of MOVING sites).
 enum { MODE_STEP = 0, MODE_STEP_MACRO = 1, MODE_REDUCE = 2, MODE_STEP_ADJ = 3 };
 
+// n / d for n < 2^31 as one high product and a shift (Granlund and Montgomery
+// 1994): with l = ceil(log2 d) and m = floor(2^(31+l) / d) + 1, m d exceeds
+// 2^(31+l) by at most 2^l, so n m / 2^(31+l) floors to n / d.  d = 1 has no
+// 32-bit m: n itself then.
+struct FastDiv {
+    unsigned m = 0, s = 0, one = 1;
+    FastDiv() = default;
+    __host__ explicit FastDiv(unsigned d)
+    {
+        if (d <= 1) return;
+        unsigned l = 0;
+        while ((1ull << l) < d) ++l;
+        m = (unsigned)((1ull << (31 + l)) / d + 1);
+        s = l - 1;
+        one = 0;
+    }
+    __device__ __forceinline__ unsigned quot(unsigned n) const { return (__umulhi(n, m) >> s) + n * one; }
+};
+
 // ---------------------------------------------------------------------------
 // Per-launch parameters.
 // ---------------------------------------------------------------------------
@@ -366,6 +385,16 @@ struct StepArgs {
     // AA variant: fin == fout is the one lattice; 0 = A-step, 1 = B-step
     int aa_phase;
     int sailfish;        // 1: rho and u summed in the Sailfish order (FP32 / FP64)
+};
+
+// One-launch iteration (step_kernel): blocks of the face rows, divisions by
+// the vectors per face row and per interior row and by the interior rows per
+// plane.  Not in StepArgs: four more fields there changed pull_kernel's
+// register allocation at its cap (16 -> 32 bytes of spills, FP16 at 512^3 8%
+// slower).
+struct StepRows {
+    unsigned face_blocks;
+    FastDiv div_face, div_row, div_plane;
 };
 
 // Initial-state kernel arguments.

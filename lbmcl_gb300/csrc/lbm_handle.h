@@ -70,8 +70,8 @@ struct lbm_handle {
     double *red_out = nullptr;
     int *status = nullptr;
     cudaStream_t stream = nullptr;
-    // the iteration graphs' second branch (face-row launches beside the
-    // interior-row launches) and its fork / join events
+    // second branch of the two-launch iterations (face rows beside interior
+    // rows) and its fork / join events
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaEvent_t ev_first = nullptr, ev_last = nullptr;
@@ -84,6 +84,8 @@ struct lbm_handle {
     unsigned grid = 0;
     // staged variant (LBM_KERNEL_STAGED)
     int kernel = LBM_KERNEL_DIRECT;
+    int step_vb = 16;         // vector bytes of the one-launch iteration; 0: two launches (step_shape)
+    unsigned step_block = 64; // threads per block of the iteration launches
     int rows = 1, gpp = 0, stages = 0;
     unsigned ngroups = 0, sgrid = 0, sblock = 0;
     size_t ssmem = 0;

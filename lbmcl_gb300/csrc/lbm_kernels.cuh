@@ -1,19 +1,21 @@
 // lbm_kernels.cuh -- the sm_103a kernels of one lattice handle.
 //
-//   pull_kernel<S, MODE>  one fused pull-stream + collide iteration
-//                         (replaces kernels.cl:321-425); MODE_REDUCE reuses
-//                         its gather to form FP64 mass / energy partials
+//   step_kernel<S, MODE>  one fused pull-stream + collide iteration
+//                         (replaces kernels.cl:321-425)
+//   pull_kernel<S, MODE>  the same in two launches (large 16-bit lattices);
+//                         MODE_REDUCE reuses its gather to form FP64 mass /
+//                         energy partials
 //   init_kernel<S>        initial state (replaces kernels.cl:277-318)
 //   dump_f_kernel<S,T>    reference post-stream buffer R_t in CSoA order
 //   load_f_kernel<S,T>    the inverse of dump_f_kernel
 //   sum_partials_kernel   deterministic final pass of the reductions
 //
-// Work decomposition of the pull kernel: one thread owns V = 16 / sizeof(S)
-// consecutive x-sites of one interior row (y, z in [1, dim-2]).  Each of the 19
-// populations is read with one aligned 16-byte load from its source row; the
+// Work decomposition: one thread owns V consecutive x-sites of one row (y, z in
+// [1, dim-2]), V sizeof(S) = 4, 8 or 16 bytes.  Each of the 19 populations is
+// read with one aligned vector load from its source row; the
 // ten populations with e_x != 0 need one more element just outside the
 // vector, read with one scalar load (the neighbouring thread's vector, so an
-// L1/L2 hit).  Results are written with one aligned 16-byte store per
+// L1/L2 hit).  Results are written with one aligned vector store per
 // population.  No shared memory, no shuffles in the step itself.
 #pragma once
 
@@ -31,38 +33,66 @@ template <class S> struct Compute { using type = float; };
 template <> struct Compute<double> { using type = double; };
 template <class S> __host__ __device__ constexpr bool is_dev16() { return sizeof(S) == 2; }
 
-// 16-byte vector load / store (ld.global.nc.v4 / st.global.v4).
-template <class S, int V>
+// Vector loads of V elements (V sizeof(S) = 2, 4, 8 or 16 bytes).  NC: the
+// read-only path (ld.global.nc), for buffers nothing writes while the kernel
+// runs.  Without it plain loads, for step_kernel, which may start before the
+// kernel that writes its input has finished (it waits for it before its first
+// load); volatile keeps them behind that wait.
+template <class S, int V, bool NC = true>
 __device__ __forceinline__ void load_vec(const S *__restrict__ p, S (&out)[V])
 {
-    static_assert(V * sizeof(S) == 16 || V * sizeof(S) == 8 || V * sizeof(S) == 4, "4-, 8- or 16-byte vectors");
-    if constexpr (V * sizeof(S) == 16) {
-        const uint4 r = __ldg(reinterpret_cast<const uint4 *>(p));
+    constexpr int B = V * (int)sizeof(S);
+    static_assert(B == 16 || B == 8 || B == 4 || B == 2, "2-, 4-, 8- or 16-byte vectors");
+    if constexpr (B == 16) {
+        uint4 r;
+        if constexpr (NC) r = __ldg(reinterpret_cast<const uint4 *>(p));
+        else asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
         memcpy(out, &r, 16);
-    } else if constexpr (V * sizeof(S) == 8) {
-        const uint2 r = __ldg(reinterpret_cast<const uint2 *>(p));
+    } else if constexpr (B == 8) {
+        uint2 r;
+        if constexpr (NC) r = __ldg(reinterpret_cast<const uint2 *>(p));
+        else asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
         memcpy(out, &r, 8);
-    } else {
-        const unsigned r = __ldg(reinterpret_cast<const unsigned *>(p));
+    } else if constexpr (B == 4) {
+        unsigned r;
+        if constexpr (NC) r = __ldg(reinterpret_cast<const unsigned *>(p));
+        else asm volatile("ld.global.u32 %0, [%1];" : "=r"(r) : "l"(p));
         memcpy(out, &r, 4);
+    } else {
+        unsigned short r;
+        if constexpr (NC) r = __ldg(reinterpret_cast<const unsigned short *>(p));
+        else asm volatile("ld.global.u16 %0, [%1];" : "=h"(r) : "l"(p));
+        memcpy(out, &r, 2);
     }
 }
 template <class S, int V>
 __device__ __forceinline__ void store_vec(S *__restrict__ p, const S (&in)[V])
 {
-    if constexpr (V * sizeof(S) == 16) {
+    constexpr int B = V * (int)sizeof(S);
+    static_assert(B == 16 || B == 8 || B == 4 || B == 2, "2-, 4-, 8- or 16-byte vectors");
+    if constexpr (B == 16) {
         uint4 r;
         memcpy(&r, in, 16);
         *reinterpret_cast<uint4 *>(p) = r;
-    } else {
+    } else if constexpr (B == 8) {
         uint2 r;
         memcpy(&r, in, 8);
         *reinterpret_cast<uint2 *>(p) = r;
+    } else if constexpr (B == 4) {
+        unsigned r;
+        memcpy(&r, in, 4);
+        *reinterpret_cast<unsigned *>(p) = r;
+    } else {
+        *p = in[0];
     }
 }
-template <class S> __device__ __forceinline__ S load_one(const S *__restrict__ p)
+template <class S, bool NC = true> __device__ __forceinline__ S load_one(const S *__restrict__ p)
 {
-    if constexpr (sizeof(S) == 2) {
+    if constexpr (!NC) {
+        S v[1];
+        load_vec<S, 1, false>(p, v);
+        return v[0];
+    } else if constexpr (sizeof(S) == 2) {
         const unsigned short v = __ldg(reinterpret_cast<const unsigned short *>(p));
         S s;
         memcpy(&s, &v, 2);
@@ -96,26 +126,27 @@ template <class S> __device__ __forceinline__ S shfl_elem(S v, int delta, bool u
 
 // Pull one population for the V sites x0..x0+V-1 of a row: the values at
 // x - EX.  `row` points at x = 0 of the source row.
-template <class S, int V, int EX>
+template <class S, int V, int EX, bool NC = true>
 __device__ __forceinline__ void gather_row(const S *__restrict__ row, int x0, int dim, S (&out)[V])
 {
     S v[V];
-    load_vec<S, V>(row + x0, v);
+    load_vec<S, V, NC>(row + x0, v);
     if constexpr (EX == 0) {
 #pragma unroll
         for (int k = 0; k < V; ++k) out[k] = v[k];
     } else if constexpr (EX == 1) {
-        out[0] = (x0 > 0) ? load_one(row + x0 - 1) : zero_elem<S>();
+        out[0] = (x0 > 0) ? load_one<S, NC>(row + x0 - 1) : zero_elem<S>();
 #pragma unroll
         for (int k = 1; k < V; ++k) out[k] = v[k - 1];
     } else {
 #pragma unroll
         for (int k = 0; k < V - 1; ++k) out[k] = v[k + 1];
-        out[V - 1] = (x0 + V < dim) ? load_one(row + x0 + V) : zero_elem<S>();
+        out[V - 1] = (x0 + V < dim) ? load_one<S, NC>(row + x0 + V) : zero_elem<S>();
     }
 }
 
 template <int V> struct MapWord;
+template <> struct MapWord<1> { using type = unsigned char; };
 template <> struct MapWord<2> { using type = unsigned short; };
 template <> struct MapWord<4> { using type = unsigned int; };
 template <> struct MapWord<8> { using type = unsigned long long; };
@@ -124,20 +155,20 @@ template <class T> __device__ __forceinline__ T nan_of();
 template <> __device__ __forceinline__ float nan_of<float>() { return __int_as_float(0x7fc00000); }
 template <> __device__ __forceinline__ double nan_of<double>() { return __longlong_as_double(0x7ff8000000000000ll); }
 
-template <class S, int V, int I>
+template <class S, int V, int I, bool NC>
 __device__ __forceinline__ void gather_pop(const S *__restrict__ fin, size_t n, size_t rowoff, int dim, int x0,
                                            S (&out)[V])
 {
     const ptrdiff_t shift = (ptrdiff_t)ez_of(I) * dim * dim + (ptrdiff_t)ey_of(I) * dim;
-    gather_row<S, V, ex_of(I)>(fin + (size_t)I * n + rowoff - shift, x0, dim, out);
+    gather_row<S, V, ex_of(I), NC>(fin + (size_t)I * n + rowoff - shift, x0, dim, out);
 }
 
-template <class S, int V, int I>
+template <class S, int V, int I, bool NC = true>
 __device__ __forceinline__ void gather_all(const S *__restrict__ fin, size_t n, size_t rowoff, int dim, int x0,
                                            S (&fs)[Q][V])
 {
-    gather_pop<S, V, I>(fin, n, rowoff, dim, x0, fs[I]);
-    if constexpr (I + 1 < Q) gather_all<S, V, I + 1>(fin, n, rowoff, dim, x0, fs);
+    gather_pop<S, V, I, NC>(fin, n, rowoff, dim, x0, fs[I]);
+    if constexpr (I + 1 < Q) gather_all<S, V, I + 1, NC>(fin, n, rowoff, dim, x0, fs);
 }
 
 // ---------------------------------------------------------------------------
@@ -621,27 +652,28 @@ __device__ __forceinline__ void update_vector(S (&fs)[Q][V], typename MapWord<V>
     const DevK K = make_devk(a.omega_f, Dev16<S>::scale, Dev16<S>::inv_scale);
     if constexpr (!DEV) {
         if (FLUID_ONLY) {
+            constexpr int P = V > 1 ? 2 : 1;  // sites per step: pairs store their moments as vectors
 #pragma unroll
-            for (int k = 0; k < V; k += 2) {
-                SiteOut o[2];
+            for (int k = 0; k < V; k += P) {
+                SiteOut o[P];
+                bool fl[P];
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
+                for (int h = 0; h < P; ++h) {
                     C f[Q];
 #pragma unroll
                     for (int i = 0; i < Q; ++i) f[i] = fs[i][k + h];
                     site_exact<C, MODE != MODE_REDUCE>(f, 0, (C)0, inv_tau, W, o[h], a.sailfish != 0);
 #pragma unroll
                     for (int i = 0; i < Q; ++i) fs[i][k + h] = f[i];
+                    // x in [2, dim-3] is FLUID; the row ends are walls / faces
+                    fl[h] = (unsigned)(x0 + k + h - 2) <= (unsigned)(dim - 5);
+                    bad |= fl[h] && o[h].bad;
+                    if (MODE == MODE_REDUCE && fl[h]) accumulate(o[h], red_m, red_e);
                 }
-                // x in [2, dim-3] is FLUID; the row ends are walls / faces
-                const bool f0 = (unsigned)(x0 + k - 2) <= (unsigned)(dim - 5);
-                const bool f1 = (unsigned)(x0 + k - 1) <= (unsigned)(dim - 5);
-                bad |= (f0 && o[0].bad) || (f1 && o[1].bad);
-                if constexpr (MODE == MODE_STEP_MACRO || MODE == MODE_STEP_ADJ)
-                    store_macro_pair<C, MODE>(a, site0 + k, f0, f1, o[0], o[1]);
-                if (MODE == MODE_REDUCE) {
-                    if (f0) accumulate(o[0], red_m, red_e);
-                    if (f1) accumulate(o[1], red_m, red_e);
+                if constexpr (MODE == MODE_STEP_MACRO || MODE == MODE_STEP_ADJ) {
+                    if constexpr (P == 2) store_macro_pair<C, MODE>(a, site0 + k, fl[0], fl[1], o[0], o[1]);
+                    else if (MODE == MODE_STEP_MACRO && fl[0]) store_macro<C>(a, site0 + k, o[0]);
+                    else if (fl[0]) store_adj<C>(a, site0 + k, o[0], false);
                 }
             }
             if (bad) atomicOr(a.status, 1);
@@ -704,7 +736,7 @@ __device__ __forceinline__ void update_vector(S (&fs)[Q][V], typename MapWord<V>
 // site's initial equilibrium w_i (kernels.cl:400-408 with the fixed
 // wall-sourced slots; interior rows are never on the lid).  Reloaded from
 // the input buffer, so the interior fast path can run on every lane first.
-template <class S, int V>
+template <class S, int V, bool NC>
 __device__ __forceinline__ void face_fix(const StepArgs &a, size_t rowoff, int xf, int k, S (&fs)[Q][V])
 {
     using C = typename Compute<S>::type;
@@ -721,13 +753,13 @@ __device__ __forceinline__ void face_fix(const StepArgs &a, size_t rowoff, int x
             else v = (S)W.w[wclass_of(j)];
         } else {
             const ptrdiff_t shift = (ptrdiff_t)ez_of(j) * dim * dim + (ptrdiff_t)ey_of(j) * dim;
-            v = load_one(fin + (size_t)j * a.n + rowoff - shift + sx);
+            v = load_one<S, NC>(fin + (size_t)j * a.n + rowoff - shift + sx);
         }
         fs[i][k] = v;
     }
 }
 
-template <class S, int MODE, int V, bool INTERIOR>
+template <class S, int MODE, int V, bool INTERIOR, bool NC = true>
 __device__ __forceinline__ void pull_vector(const StepArgs &a, int xv, int y, int z, double &red_m, double &red_e)
 {
     const int dim = a.dim;
@@ -738,12 +770,17 @@ __device__ __forceinline__ void pull_vector(const StepArgs &a, int xv, int y, in
     if (!INTERIOR) mw = __ldg(reinterpret_cast<const typename MapWord<V>::type *>(a.map + site0));
     const S *__restrict__ fin = static_cast<const S *>(a.fin);
     S fs[Q][V];
-    gather_all<S, V, 0>(fin, a.n, rowoff, dim, x0, fs);
+    gather_all<S, V, 0, NC>(fin, a.n, rowoff, dim, x0, fs);
     update_vector<S, MODE, V, INTERIOR>(fs, mw, a, y, z, x0, site0, red_m, red_e);
     if (INTERIOR && MODE != MODE_REDUCE) {
         // the walls (x = 0, dim-1) hold values nobody reads; the faces bounce back
-        if (x0 == 0) face_fix<S, V>(a, rowoff, 1, 1, fs);
-        if (x0 + V == dim) face_fix<S, V>(a, rowoff, dim - 2, V - 2, fs);
+        if constexpr (V == 1) {
+            if (x0 == 1) face_fix<S, V, NC>(a, rowoff, 1, 0, fs);
+            if (x0 == dim - 2) face_fix<S, V, NC>(a, rowoff, dim - 2, 0, fs);
+        } else {
+            if (x0 == 0) face_fix<S, V, NC>(a, rowoff, 1, 1, fs);
+            if (x0 + V == dim) face_fix<S, V, NC>(a, rowoff, dim - 2, V - 2, fs);
+        }
     }
     if (MODE != MODE_REDUCE) {
         S *__restrict__ fout = static_cast<S *>(a.fout);
@@ -753,9 +790,9 @@ __device__ __forceinline__ void pull_vector(const StepArgs &a, int xv, int y, in
 }
 
 // ---------------------------------------------------------------------------
-// Direct variant: every thread loads its V sites' populations with VB-byte
-// vector loads straight from HBM (V = VB / sizeof(S)).  One iteration is two
-// launches over disjoint sets of whole rows:
+// Every thread loads its V sites' populations with VB-byte vector loads
+// straight from HBM (V = VB / sizeof(S)).  One iteration (or reduction pass)
+// of pull_kernel is two launches over disjoint sets of whole rows:
 //   ROWS_INTERIOR  the (dim-4)^2 rows with y, z in [2, dim-3]: branch-free
 //                  FLUID update on every lane, the two x-face sites of each
 //                  row patched afterwards by face_fix (no map read)
@@ -787,32 +824,15 @@ __device__ __forceinline__ void decode_face_row(int dim, unsigned br, int &y, in
 // Launch bounds of the iteration kernels: the largest block each is compiled
 // for and the blocks of that size that must fit an SM, i.e. the register cap
 // 65536 / (threads n).  Measured at 512^3 on GB300: 16-bit storage runs
-// fastest at 128-thread blocks with three per SM (168 registers, no spills:
-// 84,448 MLUPS against 82,201 at 128 registers, which spill 88 bytes); FP32
-// with 8-byte vectors at 85 registers (256 x 3); FP64 is FP64-throughput bound
-// and left uncapped.  lbm_init clamps block_threads to max_threads.
-#ifndef LBM_MINB_16
-#define LBM_MINB_16 3
-#endif
-#ifndef LBM_MAXT_16
-#define LBM_MAXT_16 128
-#endif
-#ifndef LBM_MINB_32_V16
-#define LBM_MINB_32_V16 2
-#endif
-#ifndef LBM_MINB_32_V8
-#define LBM_MINB_32_V8 3
-#endif
-#ifndef LBM_MINB_64
-#define LBM_MINB_64 1
-#endif
+// fastest with 128 threads x 3 (168 registers: 84,448 MLUPS against 82,201 at
+// 128 registers, which spill 88 bytes); FP32 with 8-byte vectors at 85
+// registers (256 x 3); FP64 is FP64-throughput bound and left uncapped.
+// lbm_init clamps block_threads to max_threads.
+template <class S> constexpr int max_threads() { return sizeof(S) == 2 ? 128 : 256; }
 template <class S, int VB> constexpr int min_blocks()
 {
-    return sizeof(S) == 2 ? LBM_MINB_16
-         : sizeof(S) == 4 ? (VB == 16 ? LBM_MINB_32_V16 : LBM_MINB_32_V8)
-                          : LBM_MINB_64;
+    return sizeof(S) == 2 ? (VB == 16 ? 3 : VB == 8 ? 4 : 6) : sizeof(S) == 4 ? (VB == 16 ? 2 : 3) : 1;
 }
-template <class S> constexpr int max_threads() { return sizeof(S) == 2 ? LBM_MAXT_16 : 256; }
 
 template <class S, int MODE, int VB, int ROWS>
 __global__ void __launch_bounds__(max_threads<S>(), min_blocks<S, VB>()) pull_kernel(StepArgs a)
@@ -836,6 +856,55 @@ __global__ void __launch_bounds__(max_threads<S>(), min_blocks<S, VB>()) pull_ke
         pull_vector<S, MODE, V, ROWS == ROWS_INTERIOR>(a, xv, y, z, red_m, red_e);
     }
     if (MODE == MODE_REDUCE) block_reduce_write(red_m, red_e, a.partials + 2 * (size_t)a.partial_base);
+}
+
+// ---------------------------------------------------------------------------
+// One iteration over all rows in one launch: blocks [0, r.face_blocks) take
+// the face rows (they start first: their general update is the longest), the
+// others the interior rows.
+//
+// Bound: the latency of one launch and one thread's work up to about 64^3,
+// HBM above.  Two launches side by side (a fork and a join per iteration) cost
+// 2 us more per iteration at 32^3 (FP32 3.8 -> 2.9, BF16 6.0 -> 2.3) and leave
+// two last waves: FP32 200^3 188 -> 174.6, 512^3 2950 -> 2907 us (152 B a site:
+// 6.93 TB/s); only the 16-bit 16-byte-vector kernel at its register cap is
+// slower this way on large lattices (step_shape in lbm_capi.cu).  Launched as
+// a programmatic dependent of the iteration before it: its blocks may become
+// resident while that kernel's last blocks still run, and wait
+// (griddepcontrol.wait: until that kernel has completed and its stores are
+// visible) before they touch the lattices (0.1 - 0.3 us per iteration).
+// launch_dependents comes after the wait, so at most two iterations overlap.
+//
+// Face rows take two sites per thread whatever the interior's vectors: the
+// general update is long, short vectors keep its latency and registers down.
+// ---------------------------------------------------------------------------
+constexpr int FACE_VEC = 2;
+
+template <class S, int MODE, int VB>
+__global__ void __launch_bounds__(max_threads<S>(), min_blocks<S, VB>()) step_kernel(StepArgs a, StepRows r)
+{
+    constexpr int V = VB / (int)sizeof(S), VF = FACE_VEC;
+    const int dim = a.dim;
+    double red_m = 0.0, red_e = 0.0;  // unused
+    if (blockIdx.x < r.face_blocks) {
+        const unsigned g = blockIdx.x * blockDim.x + threadIdx.x;
+        const unsigned row = r.div_face.quot(g);
+        const int xv = (int)(g - row * (unsigned)(dim / VF));
+        int y, z;
+        decode_face_row(dim, row, y, z);
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;");
+        if (row < 4u * (unsigned)(dim - 3)) pull_vector<S, MODE, VF, false, false>(a, xv, y, z, red_m, red_e);
+    } else {
+        const unsigned g = (blockIdx.x - r.face_blocks) * blockDim.x + threadIdx.x;
+        const unsigned row = r.div_row.quot(g);
+        const int xv = (int)(g - row * (unsigned)(dim / V));
+        const unsigned zr = r.div_plane.quot(row);
+        const int y = 2 + (int)(row - zr * (unsigned)(dim - 4)), z = 2 + (int)zr;
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;");
+        if (z <= dim - 3) pull_vector<S, MODE, V, true, false>(a, xv, y, z, red_m, red_e);
+    }
 }
 
 // ---------------------------------------------------------------------------

@@ -9,51 +9,28 @@ namespace lbm {
 #define LBM_CAT2(a, b) a##b
 #define LBM_CAT(a, b) LBM_CAT2(a, b)
 
-// One iteration (or reduction pass) of the direct variant with VB-byte
-// vectors: the interior-row launch, then the face-row launch.  *nparts gets
-// the number of reduction partial slots the two launches use.
-// passes: bit 0 the interior-row launch, bit 1 the face-row launch (on
-// stream sf when given).
-template <int VB>
-static cudaError_t launch_direct(int mode, const StepArgs &a0, unsigned block, cudaStream_t s, unsigned *nparts,
-                                 int passes = 3, cudaStream_t sf = nullptr)
+// One iteration (or reduction pass) with 16-byte vectors as two launches: the
+// interior rows on s, the face rows on sf (s when null), so that the two can
+// run side by side.  *nparts gets the number of reduction partial slots the
+// two launches use.
+template <int MODE>
+static cudaError_t launch_rows_mode(const StepArgs &a0, unsigned block, cudaStream_t s, cudaStream_t sf,
+                                    unsigned *nparts)
 {
-    constexpr int V = VB / (int)sizeof(LBM_S);
+    constexpr int V = 16 / (int)sizeof(LBM_S);
     StepArgs a = a0;
     a.nvx = a0.dim / V;
     const size_t m = (size_t)(a.dim - 4);
     const unsigned gi = (unsigned)((m * m * (size_t)a.nvx + block - 1) / block);
     const unsigned gf = (unsigned)(((size_t)4 * (a.dim - 3) * (size_t)a.nvx + block - 1) / block);
-    for (int pass = 0; pass < 2; ++pass) {
-        if (!(passes & (1 << pass))) continue;
-        if (pass == 1 && sf) s = sf;
-        const unsigned grid = pass == 0 ? gi : gf;
-        if (grid == 0) continue;
-        a.partial_base = pass == 0 ? 0u : gi;
-        if (pass == 0) {
-            switch (mode) {
-            case MODE_STEP: pull_kernel<LBM_S, MODE_STEP, VB, ROWS_INTERIOR><<<grid, block, 0, s>>>(a); break;
-            case MODE_STEP_MACRO:
-                pull_kernel<LBM_S, MODE_STEP_MACRO, VB, ROWS_INTERIOR><<<grid, block, 0, s>>>(a);
-                break;
-            case MODE_REDUCE: pull_kernel<LBM_S, MODE_REDUCE, VB, ROWS_INTERIOR><<<grid, block, 0, s>>>(a); break;
-            case MODE_STEP_ADJ: pull_kernel<LBM_S, MODE_STEP_ADJ, VB, ROWS_INTERIOR><<<grid, block, 0, s>>>(a); break;
-            default: return cudaErrorInvalidValue;
-            }
-        } else {
-            switch (mode) {
-            case MODE_STEP: pull_kernel<LBM_S, MODE_STEP, VB, ROWS_FACES><<<grid, block, 0, s>>>(a); break;
-            case MODE_STEP_MACRO: pull_kernel<LBM_S, MODE_STEP_MACRO, VB, ROWS_FACES><<<grid, block, 0, s>>>(a); break;
-            case MODE_REDUCE: pull_kernel<LBM_S, MODE_REDUCE, VB, ROWS_FACES><<<grid, block, 0, s>>>(a); break;
-            case MODE_STEP_ADJ: pull_kernel<LBM_S, MODE_STEP_ADJ, VB, ROWS_FACES><<<grid, block, 0, s>>>(a); break;
-            default: return cudaErrorInvalidValue;
-            }
-        }
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
+    a.partial_base = 0u;
+    if (gi > 0) pull_kernel<LBM_S, MODE, 16, ROWS_INTERIOR><<<gi, block, 0, s>>>(a);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    a.partial_base = gi;
+    pull_kernel<LBM_S, MODE, 16, ROWS_FACES><<<gf, block, 0, sf ? sf : s>>>(a);
     if (nparts) *nparts = gi + gf;
-    return cudaSuccess;
+    return cudaGetLastError();
 }
 
 // One AA iteration (or reduction pass) of phase PHASE: interior rows, then
@@ -107,34 +84,70 @@ cudaError_t LBM_CAT(launch_aa_, LBM_SFX)(int mode, const StepArgs &a, unsigned b
                       : launch_aa_phase<VB, 0>(mode, a, block, s, nparts);
 }
 
-cudaError_t LBM_CAT(launch_pull_, LBM_SFX)(int mode, const StepArgs &a, unsigned block, cudaStream_t s,
-                                           unsigned *nparts)
+cudaError_t LBM_CAT(launch_reduce_, LBM_SFX)(const StepArgs &a, unsigned block, cudaStream_t s, unsigned *nparts)
 {
-    return launch_direct<16>(mode, a, block, s, nparts);
+    return launch_rows_mode<MODE_REDUCE>(a, block, s, nullptr, nparts);
 }
 
-// One iteration (MODE_STEP or MODE_STEP_ADJ) of the direct variant (VB =
-// 16) or the narrow one (VB = 8) with the face-row launch on stream sf, so
-// that the two launches can run side by side.
-cudaError_t LBM_CAT(launch_split_, LBM_SFX)(int vb, int mode, const StepArgs &a, unsigned block, cudaStream_t s,
-                                            cudaStream_t sf)
+// 16-bit storage only (large lattices; see step_shape in lbm_capi.cu).
+cudaError_t LBM_CAT(launch_rows_, LBM_SFX)(int mode, const StepArgs &a, unsigned block, cudaStream_t s,
+                                           cudaStream_t sf)
 {
-    if (mode != MODE_STEP && mode != MODE_STEP_ADJ) return cudaErrorInvalidValue;
-    if (vb == 16) return launch_direct<16>(mode, a, block, s, nullptr, 3, sf);
-    if constexpr (sizeof(LBM_S) < 8) {
-        if (vb == 8) return launch_direct<8>(mode, a, block, s, nullptr, 3, sf);
+    if constexpr (sizeof(LBM_S) == 2) {
+        switch (mode) {
+        case MODE_STEP: return launch_rows_mode<MODE_STEP>(a, block, s, sf, nullptr);
+        case MODE_STEP_MACRO: return launch_rows_mode<MODE_STEP_MACRO>(a, block, s, sf, nullptr);
+        case MODE_STEP_ADJ: return launch_rows_mode<MODE_STEP_ADJ>(a, block, s, sf, nullptr);
+        }
     }
     return cudaErrorInvalidValue;
 }
 
-cudaError_t LBM_CAT(launch_narrow_, LBM_SFX)(int mode, const StepArgs &a, unsigned block, cudaStream_t s)
+// One iteration with VB-byte vectors in one launch, as a programmatic
+// dependent of the launch before it on the stream.
+template <int VB, int MODE>
+static cudaError_t launch_step_mode(const StepArgs &a, unsigned block, cudaStream_t s)
 {
-    if constexpr (sizeof(LBM_S) < 8) {
-        if (mode == MODE_REDUCE) return cudaErrorInvalidValue;
-        return launch_direct<8>(mode, a, block, s, nullptr);
-    } else {
-        return cudaErrorInvalidValue;  // one double per 8 bytes: no narrow variant
+    constexpr unsigned V = VB / (int)sizeof(LBM_S), VF = FACE_VEC;
+    const unsigned dim = (unsigned)a.dim, m = dim - 4;
+    const size_t ni = (size_t)m * m * (dim / V), nf = (size_t)4 * (dim - 3) * (dim / VF);
+    if (ni >> 31) return cudaErrorInvalidValue;  // FastDiv's range
+    StepRows r;
+    r.face_blocks = (unsigned)((nf + block - 1) / block);
+    r.div_face = FastDiv(dim / VF);
+    r.div_row = FastDiv(dim / V);
+    r.div_plane = FastDiv(m);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(r.face_blocks + (unsigned)((ni + block - 1) / block));
+    lc.blockDim = dim3(block);
+    lc.stream = s;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, step_kernel<LBM_S, MODE, VB>, a, r);
+}
+
+template <int VB> static cudaError_t launch_step_vb(int mode, const StepArgs &a, unsigned block, cudaStream_t s)
+{
+    switch (mode) {
+    case MODE_STEP: return launch_step_mode<VB, MODE_STEP>(a, block, s);
+    case MODE_STEP_MACRO: return launch_step_mode<VB, MODE_STEP_MACRO>(a, block, s);
+    case MODE_STEP_ADJ: return launch_step_mode<VB, MODE_STEP_ADJ>(a, block, s);
+    default: return cudaErrorInvalidValue;
     }
+}
+
+cudaError_t LBM_CAT(launch_step_, LBM_SFX)(int vb, int mode, const StepArgs &a, unsigned block, cudaStream_t s)
+{
+    switch (vb) {
+    case 16: return launch_step_vb<16>(mode, a, block, s);
+    case 8: return launch_step_vb<8>(mode, a, block, s);
+    case 4:
+        if constexpr (sizeof(LBM_S) < 8) return launch_step_vb<4>(mode, a, block, s);
+    }
+    return cudaErrorInvalidValue;
 }
 
 cudaError_t LBM_CAT(launch_staged_, LBM_SFX)(int mode, const StepArgs &a, unsigned grid, unsigned block,

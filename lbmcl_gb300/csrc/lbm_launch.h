@@ -13,11 +13,12 @@ struct DumpArgs;
 
 // prec: 0 FP32, 1 FP64, 2 FP16, 3 BF16 (lbm_precision)
 #define LBM_DECLARE_LAUNCHERS(SFX)                                                                   \
-    cudaError_t launch_pull_##SFX(int mode, const StepArgs &a, unsigned block, cudaStream_t s,       \
-                                  unsigned *nparts);                                                 \
-    cudaError_t launch_narrow_##SFX(int mode, const StepArgs &a, unsigned block, cudaStream_t s);    \
-    cudaError_t launch_split_##SFX(int vb, int mode, const StepArgs &a, unsigned block, cudaStream_t s,\
-                                   cudaStream_t sf);                                                 \
+    cudaError_t launch_reduce_##SFX(const StepArgs &a, unsigned block, cudaStream_t s,               \
+                                    unsigned *nparts);                                               \
+    cudaError_t launch_rows_##SFX(int mode, const StepArgs &a, unsigned block, cudaStream_t s,       \
+                                  cudaStream_t sf);                                                  \
+    cudaError_t launch_step_##SFX(int vb, int mode, const StepArgs &a, unsigned block,               \
+                                  cudaStream_t s);                                                   \
     cudaError_t launch_aa_##SFX(int mode, const StepArgs &a, unsigned block, cudaStream_t s,         \
                                 unsigned *nparts);                                                   \
     cudaError_t launch_staged_##SFX(int mode, const StepArgs &a, unsigned grid, unsigned block,      \
