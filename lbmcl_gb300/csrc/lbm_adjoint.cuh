@@ -44,13 +44,10 @@ struct AdjArgs {
     const void *target;  // loss: u_x target on the plane, adjoint type, [x + z*dim]
     double *loss_part;   // loss: per block partial sums
     int dim;
-    int nvx;
-    unsigned nvec;
     size_t n;
     double omega;        // 1/tau in the forward's precision
     double dloss;        // loss-gradient seed scale (dJ/dL * 2 / M)
     int plane_y;         // loss plane
-    unsigned tau_base;   // first tau_acc slot of this launch
 };
 
 template <class S> struct AdjType { using type = float; };
@@ -122,12 +119,21 @@ __device__ __forceinline__ void adjoint_moving(const A (&g)[Q], A (&b)[Q], A lid
     adjoint_moving_rho<A>(b, rho, lid, dlid);
 }
 
-// FLUID adjoint written around opposite pairs (i, i') with e_i.u = +-a:
-//   p_(+-) = base +- 3a, base = 1 + 4.5 a^2 - 1.5 u^2
-//   B0 = sum_c w_c sum_pairs (s base + 3 a d),   s = b+ + b-, d = b+ - b-
-//   G  = sum_c w_c sum_pairs e_i (3 d + 9 a s) - 3 u SB,  SB = sum_c w_c sum s
-//   a_(+-) = (1 - omega) b_(+-) + omega (B0 - G.u) +- omega G.e_i
-//   dJ/domega += rho B0 - sum_i b_i g_i
+// FLUID adjoint written around opposite pairs (i, i') with 3 e_i.u = +-m,
+// s = b+ + b-, d = b+ - b-.  Every weighted sum the formulas above need reduces
+// to three kinds (c: weight class):
+//   S = sum_i w_i b_i,  K = sum_c w_c sum_pairs m^2 s,
+//   g = sum_c w_c sum_pairs e_i (d + m s) - u S          (G = 3 g)
+//   B0 - G.u = (1 + 1.5 u^2) S - K / 2
+//   a_(+-) = (1 - omega) b_(+-) + omega (B0 - G.u) +- 3 omega g.e_i
+// (the 4.5 a^2 terms of B0 and the 9 a^2 terms of G.u are both multiples of K,
+// the linear ones cancel): about 145 operations a site instead of 200 for
+// forming B0 and G separately.  The tau term rho B0 - sum_i b_i g_i takes B0
+// from its own definition, sum_i b_i w_i p_i (45 operations more, full-state
+// sweeps only): two large sums cancel there, and the gradient keeps the value
+// it has in that form (rewritten about the rest state, or with B0 from S, K
+// and g, dJ/dtau moves by up to 1e-6 of itself, no closer to 64 bits: the
+// rounding of the forward's trajectory dominates its error).
 // e_i . u as a signed sum of the non-zero terms (chosen at compile time: no
 // multiplications by the 0 / +-1 components)
 template <class A> __device__ __forceinline__ A proj_sum(int i, A ux, A uy, A uz)
@@ -140,50 +146,53 @@ template <class A> __device__ __forceinline__ A proj_sum(int i, A ux, A uy, A uz
     return s;
 }
 
+// Returns B0.
 template <class A>
 __device__ __forceinline__ A adjoint_fluid_core(A (&b)[Q], A ux, A uy, A uz, A omega)
 {
     const A c0 = (A)1 - (A)1.5 * (ux * ux + uy * uy + uz * uz);
-    // per weight class accumulators: rest (0), axis (1), edge (2)
-    A B[3] = {b[0] * c0, 0, 0}, SB[3] = {b[0], 0, 0};
-    A Gx[3] = {0, 0, 0}, Gy[3] = {0, 0, 0}, Gz[3] = {0, 0, 0};
+    A B[3] = {b[0] * c0, 0, 0};
+    const A x3 = (A)3 * ux, y3 = (A)3 * uy, z3 = (A)3 * uz;
+    // per weight class accumulators: axis (1), edge (2)
+    A S[3] = {b[0], 0, 0}, K[3] = {0, 0, 0}, Gx[3] = {0, 0, 0}, Gy[3] = {0, 0, 0}, Gz[3] = {0, 0, 0};
     // (i, i') pairs with e_i listed first
     constexpr int P[9][2] = {{1, 3}, {2, 4}, {6, 5}, {7, 9}, {8, 10}, {11, 17}, {12, 18}, {15, 13}, {16, 14}};
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
         const int i = P[k][0], j = P[k][1];
         const int c = wclass_of(i);
-        const A aa = proj_sum<A>(i, ux, uy, uz);
+        const A m = proj_sum<A>(i, x3, y3, z3);
         const A sm = b[i] + b[j], df = b[i] - b[j];
+        const A aa = proj_sum<A>(i, ux, uy, uz);
         B[c] += sm * (c0 + (A)4.5 * aa * aa) + (A)3 * aa * df;
-        SB[c] += sm;
-        const A q = (A)3 * df + (A)9 * aa * sm;
+        const A ms = m * sm;
+        const A q = df + ms;
+        S[c] += sm;
+        K[c] += m * ms;
         if (ex_of(i)) Gx[c] += ex_of(i) > 0 ? q : -q;
         if (ey_of(i)) Gy[c] += ey_of(i) > 0 ? q : -q;
         if (ez_of(i)) Gz[c] += ez_of(i) > 0 ? q : -q;
     }
     // class weights: rest, axis (population 1), edge (population 7)
     const A w0 = w_of<A>(0), w1 = w_of<A>(1), w2 = w_of<A>(7);
-    const A B0 = w0 * B[0] + w1 * B[1] + w2 * B[2];
-    const A sb = w0 * SB[0] + w1 * SB[1] + w2 * SB[2];
-    const A gx = w1 * Gx[1] + w2 * Gx[2] - (A)3 * ux * sb;
-    const A gy = w1 * Gy[1] + w2 * Gy[2] - (A)3 * uy * sb;
-    const A gz = w1 * Gz[1] + w2 * Gz[2] - (A)3 * uz * sb;
-    const A keep = (A)1 - omega;
-    const A oc = omega * (B0 - (gx * ux + gy * uy + gz * uz));
+    const A sb = w0 * S[0] + w1 * S[1] + w2 * S[2];
+    const A gx = w1 * Gx[1] + w2 * Gx[2] - ux * sb;
+    const A gy = w1 * Gy[1] + w2 * Gy[2] - uy * sb;
+    const A gz = w1 * Gz[1] + w2 * Gz[2] - uz * sb;
+    const A u2 = ux * ux + uy * uy + uz * uz;
+    const A o = (sb + (A)1.5 * u2 * sb) - (A)0.5 * (w1 * K[1] + w2 * K[2]);  // B0 - G.u
+    // omega (3 g), not (3 omega) g: a rounded 3 omega would bias every step alike
+    const A keep = (A)1 - omega, oc = omega * o;
+    const A tx = omega * ((A)3 * gx), ty = omega * ((A)3 * gy), tz = omega * ((A)3 * gz);
     b[0] = keep * b[0] + oc;
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
         const int i = P[k][0], j = P[k][1];
-        A ge = 0;
-        if (ex_of(i)) ge += ex_of(i) > 0 ? gx : -gx;
-        if (ey_of(i)) ge += ey_of(i) > 0 ? gy : -gy;
-        if (ez_of(i)) ge += ez_of(i) > 0 ? gz : -gz;
-        const A t = omega * ge;
+        const A t = proj_sum<A>(i, tx, ty, tz);
         b[i] = keep * b[i] + (oc + t);
         b[j] = keep * b[j] + (oc - t);
     }
-    return B0;
+    return w0 * B[0] + w1 * B[1] + w2 * B[2];
 }
 
 // A FLUID site's pre-collision populations g (adjoint type) and its moments
@@ -307,135 +316,178 @@ __device__ __forceinline__ void adjoint_face_fix(const AdjArgs &a, size_t rowoff
     for (int j = 0; j < Q; ++j) {
         const int o = opp_of(j);
         const ptrdiff_t shift = (ptrdiff_t)ez_of(j) * dim * dim + (ptrdiff_t)ey_of(j) * dim;
-        bs[j][k] = load_one(ain + (size_t)o * a.n + rowoff - shift + (xf - ex_of(j)));
+        bs[j][k] = load_one<A, false>(ain + (size_t)o * a.n + rowoff - shift + (xf - ex_of(j)));
     }
 }
 
-// One adjoint step a_{k+1} -> a_k over the rows of one kind (ROWS_INTERIOR:
-// y, z in [2, dim-3], branch-free FLUID adjoint then the row ends patched;
-// ROWS_FACES: the general path).  V = VB / sizeof(A) sites per thread.
-// register cap of the adjoint kernels: 128 (two 256-thread blocks per SM)
-// for the FP32 adjoint, uncapped for FP64
-#ifndef LBM_ADJ_MINB
-#define LBM_ADJ_MINB 2
-#endif
+// vector bytes of the one-step kernel: two FP32 sites or one FP64 site per thread
+constexpr int ADJ_VB = 8;
 
+// One adjoint step a_{k+1} -> a_k for the V sites x0 .. x0 + V - 1 of row
+// (y, z): INTERIOR (y, z in [2, dim-3]): branch-free FLUID adjoint, then the
+// row ends patched; else the general, map-driven path.  dw += their tau term.
 // MACRO = false: a.fwd is the forward state Q_k (its pull gives the
 // pre-collision populations); MACRO = true: a.fwd holds the three planes the
 // MODE_STEP_ADJ iteration from Q_k stored (compute type), and no tau term is
 // formed.
-template <class S, class A, int VB, int ROWS, bool MACRO>
-__global__ void __launch_bounds__(256, sizeof(A) == 8 ? 1 : LBM_ADJ_MINB) adjoint_kernel(AdjArgs a)
+template <class S, class A, int V, bool INTERIOR, bool MACRO>
+__device__ __forceinline__ void adjoint_vector(const AdjArgs &a, int xv, int y, int z, A &dw)
 {
     using C = typename Compute<S>::type;
-    constexpr int V = VB / (int)sizeof(A);
     const int dim = a.dim;
-    const int nvx = dim / V;
-    const unsigned nrows = ROWS == ROWS_INTERIOR ? (unsigned)(dim - 4) * (unsigned)(dim - 4) : 4u * (unsigned)(dim - 3);
-    const unsigned g0 = blockIdx.x * blockDim.x + threadIdx.x;
-    A dw = 0;
-    if (g0 < nrows * (unsigned)nvx) {
-        const unsigned row = g0 / (unsigned)nvx;
-        const int xv = (int)(g0 - row * (unsigned)nvx);
-        int y, z;
-        if (ROWS == ROWS_INTERIOR) {
-            y = 2 + (int)(row % (unsigned)(dim - 4));
-            z = 2 + (int)(row / (unsigned)(dim - 4));
-        } else {
-            decode_face_row(dim, row, y, z);
-        }
-        const int x0 = xv * V;
-        const size_t rowoff = (size_t)z * dim * dim + (size_t)y * dim;
-        const size_t site0 = rowoff + (size_t)x0;
+    const int x0 = xv * V;
+    const size_t rowoff = (size_t)z * dim * dim + (size_t)y * dim;
+    const size_t site0 = rowoff + (size_t)x0;
 
-        // reverse streaming: slot i of site s takes a_{k+1}(s + e_i, i)
-        const A *ain = static_cast<const A *>(a.ain);
-        A bs[Q][V];
+    // reverse streaming: slot i of site s takes a_{k+1}(s + e_i, i)
+    const A *ain = static_cast<const A *>(a.ain);
+    A bs[Q][V];
 #pragma unroll
-        for (int i = 0; i < Q; ++i) {
-            const ptrdiff_t shift = (ptrdiff_t)ez_of(i) * dim * dim + (ptrdiff_t)ey_of(i) * dim;
-            const A *src = ain + (size_t)i * a.n + rowoff + shift;
-            if (ex_of(i) == 1) gather_row<A, V, -1>(src, x0, dim, bs[i]);
-            else if (ex_of(i) == -1) gather_row<A, V, 1>(src, x0, dim, bs[i]);
-            else gather_row<A, V, 0>(src, x0, dim, bs[i]);
-        }
-        const A omega = (A)a.omega;
-        // forward values: the pulled populations R_k(s), or the stored
-        // linearisation point (three planes, same element type as A)
-        S fsv[MACRO ? 1 : Q][MACRO ? 1 : V];
-        C mv[MACRO ? 3 : 1][MACRO ? V : 1];
-        if constexpr (MACRO) {
-            const C *m = static_cast<const C *>(a.fwd);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) load_vec<C, V>(m + (size_t)c * a.n + site0, mv[c]);
-        } else {
-            const S *fwd = static_cast<const S *>(a.fwd);
-            gather_all<S, V, 0>(fwd, a.n, rowoff, dim, x0, fsv);
-        }
-
-        if (ROWS == ROWS_INTERIOR) {
-#pragma unroll
-            for (int k = 0; k < V; ++k) {
-                A b[Q];
-#pragma unroll
-                for (int i = 0; i < Q; ++i) b[i] = bs[i][k];
-                if constexpr (MACRO) {
-                    adjoint_fluid_core<A>(b, (A)mv[0][k], (A)mv[1][k], (A)mv[2][k], omega);
-                } else {
-                    S v[Q];
-#pragma unroll
-                    for (int i = 0; i < Q; ++i) v[i] = fsv[i][k];
-                    A g[Q], rho, ux, uy, uz;
-                    forward_point<S, A>(v, g, rho, ux, uy, uz);
-                    A d = 0;
-                    adjoint_fluid_point<A>(g, b, rho, ux, uy, uz, omega, d);
-                    // x in [2, dim-3] is FLUID; the row ends are patched below
-                    if ((unsigned)(x0 + k - 2) <= (unsigned)(dim - 5)) dw += d;
-                }
-#pragma unroll
-                for (int i = 0; i < Q; ++i) bs[i][k] = b[i];
-            }
-            if (x0 == 0) {
-#pragma unroll
-                for (int i = 0; i < Q; ++i) bs[i][0] = (A)0;
-                adjoint_face_fix<A, V>(a, rowoff, 1, 1, bs);
-            }
-            if (x0 + V == dim) {
-#pragma unroll
-                for (int i = 0; i < Q; ++i) bs[i][V - 1] = (A)0;
-                adjoint_face_fix<A, V>(a, rowoff, dim - 2, V - 2, bs);
-            }
-        } else {
-            const typename MapWord<V>::type mw =
-                __ldg(reinterpret_cast<const typename MapWord<V>::type *>(a.map + site0));
-            const C *lid = static_cast<const C *>(a.lid);
-            const Weights<C> W = make_weights<C>();
-#pragma unroll
-            for (int k = 0; k < V; ++k) {
-                const uint8_t b8 = (uint8_t)(mw >> (8 * k));
-                A b[Q];
-#pragma unroll
-                for (int i = 0; i < Q; ++i) b[i] = bs[i][k];
-                const C lidv = (b8 & M_FRONT) ? lid[(size_t)y * dim + x0 + k] : (C)0;
-                A dl = 0;
-                if constexpr (MACRO) {
-                    adjoint_site_macro<A>(b, b8, (A)mv[0][k], (A)mv[1][k], (A)mv[2][k], (A)lidv, omega, dl);
-                } else {
-                    S v[Q];
-#pragma unroll
-                    for (int i = 0; i < Q; ++i) v[i] = fsv[i][k];
-                    adjoint_general<S, A, C>(v, b, b8, lidv, omega, W, dw, dl);
-                }
-                if (b8 == M_FRONT) a.grad_lid[(size_t)y * dim + x0 + k] += (double)dl;
-#pragma unroll
-                for (int i = 0; i < Q; ++i) bs[i][k] = b[i];
-            }
-        }
-        A *aout = static_cast<A *>(a.aout);
-#pragma unroll
-        for (int i = 0; i < Q; ++i) store_vec<A, V>(aout + (size_t)i * a.n + site0, bs[i]);
+    for (int i = 0; i < Q; ++i) {
+        const ptrdiff_t shift = (ptrdiff_t)ez_of(i) * dim * dim + (ptrdiff_t)ey_of(i) * dim;
+        const A *src = ain + (size_t)i * a.n + rowoff + shift;
+        if (ex_of(i) == 1) gather_row<A, V, -1, false>(src, x0, dim, bs[i]);
+        else if (ex_of(i) == -1) gather_row<A, V, 1, false>(src, x0, dim, bs[i]);
+        else gather_row<A, V, 0, false>(src, x0, dim, bs[i]);
     }
-    if constexpr (!MACRO) block_reduce_add((double)dw, a.tau_acc + a.tau_base);
+    const A omega = (A)a.omega;
+    // forward values: the pulled populations R_k(s), or the stored
+    // linearisation point (three planes, same element type as A)
+    S fsv[MACRO ? 1 : Q][MACRO ? 1 : V];
+    C mv[MACRO ? 3 : 1][MACRO ? V : 1];
+    if constexpr (MACRO) {
+        const C *m = static_cast<const C *>(a.fwd);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) load_vec<C, V, false>(m + (size_t)c * a.n + site0, mv[c]);
+    } else {
+        const S *fwd = static_cast<const S *>(a.fwd);
+        gather_all<S, V, 0, false>(fwd, a.n, rowoff, dim, x0, fsv);
+    }
+
+    if constexpr (INTERIOR) {
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+            A b[Q];
+#pragma unroll
+            for (int i = 0; i < Q; ++i) b[i] = bs[i][k];
+            if constexpr (MACRO) {
+                adjoint_fluid_core<A>(b, (A)mv[0][k], (A)mv[1][k], (A)mv[2][k], omega);
+            } else {
+                S v[Q];
+#pragma unroll
+                for (int i = 0; i < Q; ++i) v[i] = fsv[i][k];
+                A g[Q], rho, ux, uy, uz;
+                forward_point<S, A>(v, g, rho, ux, uy, uz);
+                A d = 0;
+                adjoint_fluid_point<A>(g, b, rho, ux, uy, uz, omega, d);
+                // x in [2, dim-3] is FLUID; the row ends are patched below
+                if ((unsigned)(x0 + k - 2) <= (unsigned)(dim - 5)) dw += d;
+            }
+#pragma unroll
+            for (int i = 0; i < Q; ++i) bs[i][k] = b[i];
+        }
+        if (x0 == 0) {
+#pragma unroll
+            for (int i = 0; i < Q; ++i) bs[i][0] = (A)0;
+        }
+        if (x0 + V == dim) {
+#pragma unroll
+            for (int i = 0; i < Q; ++i) bs[i][V - 1] = (A)0;
+        }
+        constexpr int K1 = V > 1 ? 1 : 0, K2 = V > 1 ? V - 2 : 0;  // x-face sites within their vectors
+        if (x0 + K1 == 1) adjoint_face_fix<A, V>(a, rowoff, 1, K1, bs);
+        if (x0 + K2 == dim - 2) adjoint_face_fix<A, V>(a, rowoff, dim - 2, K2, bs);
+    } else {
+        const typename MapWord<V>::type mw = __ldg(reinterpret_cast<const typename MapWord<V>::type *>(a.map + site0));
+        const C *lid = static_cast<const C *>(a.lid);
+        const Weights<C> W = make_weights<C>();
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+            const uint8_t b8 = (uint8_t)(mw >> (8 * k));
+            A b[Q];
+#pragma unroll
+            for (int i = 0; i < Q; ++i) b[i] = bs[i][k];
+            const C lidv = (b8 & M_FRONT) ? lid[(size_t)y * dim + x0 + k] : (C)0;
+            A dl = 0;
+            if constexpr (MACRO) {
+                adjoint_site_macro<A>(b, b8, (A)mv[0][k], (A)mv[1][k], (A)mv[2][k], (A)lidv, omega, dl);
+            } else {
+                S v[Q];
+#pragma unroll
+                for (int i = 0; i < Q; ++i) v[i] = fsv[i][k];
+                adjoint_general<S, A, C>(v, b, b8, lidv, omega, W, dw, dl);
+            }
+            if (b8 == M_FRONT) a.grad_lid[(size_t)y * dim + x0 + k] += (double)dl;
+#pragma unroll
+            for (int i = 0; i < Q; ++i) bs[i][k] = b[i];
+        }
+    }
+    A *aout = static_cast<A *>(a.aout);
+#pragma unroll
+    for (int i = 0; i < Q; ++i) store_vec<A, V>(aout + (size_t)i * a.n + site0, bs[i]);
+}
+
+// One adjoint step over all rows in one launch, the face rows' blocks first,
+// a programmatic dependent of the launch before it (see step_kernel).  Bound:
+// HBM on lattices beyond L2 (164 B a site with stored points, 190 with full
+// 16-bit states), launch and one thread's latency below.  us per backward
+// iteration with stored points, two launches -> one: 32^3 6.0 -> 3.4, 64^3
+// 14.4 -> 7.1, 96^3 32 -> 22.6, 128^3 (FP16; from two steps per launch) 58.7
+// -> 51.4.  One site per thread instead of two: 64^3 7.2, 128^3 54.6, 256^3
+// 413 against 393.
+template <class S, class A, bool MACRO>
+__global__ void __launch_bounds__(256, sizeof(A) == 8 ? 1 : 2) adjoint_kernel(AdjArgs a, StepRows r)
+{
+    constexpr int V = ADJ_VB / (int)sizeof(A);
+    const int dim = a.dim;
+    A dw = 0;
+    if (blockIdx.x < r.face_blocks) {
+        const unsigned g = blockIdx.x * blockDim.x + threadIdx.x;
+        const unsigned row = r.div_face.quot(g);
+        const int xv = (int)(g - row * (unsigned)(dim / V));
+        int y, z;
+        decode_face_row(dim, row, y, z);
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;");
+        if (row < 4u * (unsigned)(dim - 3)) adjoint_vector<S, A, V, false, MACRO>(a, xv, y, z, dw);
+    } else {
+        const unsigned g = (blockIdx.x - r.face_blocks) * blockDim.x + threadIdx.x;
+        const unsigned row = r.div_row.quot(g);
+        const int xv = (int)(g - row * (unsigned)(dim / V));
+        const unsigned zr = r.div_plane.quot(row);
+        const int y = 2 + (int)(row - zr * (unsigned)(dim - 4)), z = 2 + (int)zr;
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;");
+        if (z <= dim - 3) adjoint_vector<S, A, V, true, MACRO>(a, xv, y, z, dw);
+    }
+    if constexpr (!MACRO) block_reduce_add(dw, a.tau_acc);
+}
+
+// blocks of a one-step launch with V sites per thread
+inline unsigned adjoint_blocks(int dim, int V, unsigned block, unsigned *face)
+{
+    const size_t nvx = (size_t)(dim / V), m = (size_t)(dim - 4);
+    *face = (unsigned)((4 * (size_t)(dim - 3) * nvx + block - 1) / block);
+    return *face + (unsigned)((m * m * nvx + block - 1) / block);
+}
+
+template <class S, class A, bool MACRO>
+cudaError_t launch_adjoint_kernel(const AdjArgs &a, unsigned block, cudaStream_t s)
+{
+    constexpr int V = ADJ_VB / (int)sizeof(A);
+    StepRows r;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(adjoint_blocks(a.dim, V, block, &r.face_blocks));
+    lc.blockDim = dim3(block);
+    lc.stream = s;
+    r.div_face = r.div_row = FastDiv((unsigned)(a.dim / V));
+    r.div_plane = FastDiv((unsigned)(a.dim - 4));
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, adjoint_kernel<S, A, MACRO>, a, r);
 }
 
 // ---------------------------------------------------------------------------
@@ -735,7 +787,7 @@ __global__ void __launch_bounds__(ADJ2_EX * adj2_ey<MACRO>(), MACRO ? LBM_ADJ2M_
     }
     // one MOVING site per column, in one chunk: a single writer per column
     if (owned && zi0 <= dim - 2 && dim - 2 < zi1) a.grad_lid[col] += (double)dl;
-    if constexpr (!MACRO) block_reduce_add((double)dw, a.tau_acc);
+    if constexpr (!MACRO) block_reduce_add(dw, a.tau_acc);
 }
 
 // ---------------------------------------------------------------------------
@@ -1034,8 +1086,7 @@ __global__ void export_adjoint_kernel(const A *__restrict__ adj, T *__restrict__
 
 // Launchers of the FP64 adjoint over FP32 / 16-bit storage (their own
 // translation unit, lbm_adjoint_f64.cu): prec is the storage lbm_precision.
-cudaError_t launch_adjoint_step_a64(int prec, const AdjArgs &a, unsigned gi, unsigned gf, unsigned block,
-                                    cudaStream_t s, bool macro);
+cudaError_t launch_adjoint_step_a64(int prec, const AdjArgs &a, unsigned block, cudaStream_t s, bool macro);
 cudaError_t launch_loss_seed_a64(int prec, const AdjArgs &a, unsigned grid, unsigned block, cudaStream_t s);
 cudaError_t launch_lid_init_grad_a64(int prec, const AdjArgs &a, cudaStream_t s);
 

@@ -9,36 +9,20 @@
 namespace lbm {
 namespace {
 
-template <class S, bool MACRO>
-cudaError_t step_a64(const AdjArgs &a0, unsigned gi, unsigned gf, unsigned block, cudaStream_t s)
+template <class S> cudaError_t step_a64(const AdjArgs &a, unsigned block, cudaStream_t s, bool macro)
 {
-    AdjArgs a = a0;
-    if (gi > 0) {
-        a.tau_base = 0;
-        adjoint_kernel<S, double, 16, ROWS_INTERIOR, MACRO><<<gi, block, 0, s>>>(a);
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
-    a.tau_base = gi;
-    adjoint_kernel<S, double, 16, ROWS_FACES, MACRO><<<gf, block, 0, s>>>(a);
-    return cudaGetLastError();
-}
-
-template <class S>
-cudaError_t step_any(const AdjArgs &a, unsigned gi, unsigned gf, unsigned block, cudaStream_t s, bool macro)
-{
-    return macro ? step_a64<S, true>(a, gi, gf, block, s) : step_a64<S, false>(a, gi, gf, block, s);
+    return macro ? launch_adjoint_kernel<S, double, true>(a, block, s)
+                 : launch_adjoint_kernel<S, double, false>(a, block, s);
 }
 
 }  // namespace
 
-cudaError_t launch_adjoint_step_a64(int prec, const AdjArgs &a, unsigned gi, unsigned gf, unsigned block,
-                                    cudaStream_t s, bool macro)
+cudaError_t launch_adjoint_step_a64(int prec, const AdjArgs &a, unsigned block, cudaStream_t s, bool macro)
 {
     switch (prec) {
-    case LBM_FP32: return step_any<float>(a, gi, gf, block, s, macro);
-    case LBM_FP16: return step_any<__half>(a, gi, gf, block, s, macro);
-    case LBM_BF16: return step_any<__nv_bfloat16>(a, gi, gf, block, s, macro);
+    case LBM_FP32: return step_a64<float>(a, block, s, macro);
+    case LBM_FP16: return step_a64<__half>(a, block, s, macro);
+    case LBM_BF16: return step_a64<__nv_bfloat16>(a, block, s, macro);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -58,16 +58,17 @@ int fail(int code, const char *fmt, ...)
 // FP64 adjoint arithmetic: FP64 storage, or asked for (lbm_config.adjoint_fp64)
 bool adj64(const lbm_t *h) { return h->prec == LBM_FP64 || h->cfg.adjoint_fp64 != 0; }
 size_t adj_bytes(const lbm_t *h) { return adj64(h) ? 8 : 4; }
-// adjoint kernels: 2 sites per thread (8-byte FP32 / 16-byte FP64 vectors)
-constexpr int kAdjV = 2;
+// Sites per thread of the one-step adjoint kernel: two for FP32 (8-byte
+// vectors), one for FP64 (its time is the FP64 pipe's, and two sites take 230
+// registers or more: 64^3 FP64 storage, backward 105 us per iteration with two
+// launches of two sites, 70 with one of one).
+int adj_vec(const lbm_t *h) { return adj64(h) ? 1 : 2; }
 
-// blocks of the interior-row and face-row adjoint launches
-void adj_grids(const lbm_t *h, unsigned &gi, unsigned &gf)
+// blocks of its launch
+unsigned adj_grid(const lbm_t *h)
 {
-    const size_t nvx = (size_t)(h->dim / kAdjV);
-    const size_t m = (size_t)(h->dim - 4);
-    gi = (unsigned)((m * m * nvx + kAdjBlock - 1) / kAdjBlock);
-    gf = (unsigned)((4 * (size_t)(h->dim - 3) * nvx + kAdjBlock - 1) / kAdjBlock);
+    unsigned face;
+    return lbm::adjoint_blocks(h->dim, adj_vec(h), kAdjBlock, &face);
 }
 
 lbm::AdjArgs adj_args(const lbm_t *h)
@@ -79,29 +80,18 @@ lbm::AdjArgs adj_args(const lbm_t *h)
     a.tau_acc = h->adj.tau_acc;
     a.target = h->adj.target;
     a.dim = h->dim;
-    a.nvx = h->dim / kAdjV;
-    a.nvec = (unsigned)((size_t)a.nvx * (size_t)(h->dim - 2) * (size_t)(h->dim - 2));
     a.n = h->n;
     a.omega = h->inv_tau;
     a.plane_y = h->adj.plane_y;
     return a;
 }
 
-template <class S, bool MACRO>
-cudaError_t run_adjoint_step(const lbm::AdjArgs &a0, unsigned gi, unsigned gf, cudaStream_t s)
+template <class S>
+cudaError_t run_adjoint_step(const lbm::AdjArgs &a, cudaStream_t s, bool macro)
 {
     using A = typename lbm::AdjType<S>::type;
-    constexpr int VB = kAdjV * (int)sizeof(A);
-    lbm::AdjArgs a = a0;
-    if (gi > 0) {
-        a.tau_base = 0;
-        lbm::adjoint_kernel<S, A, VB, lbm::ROWS_INTERIOR, MACRO><<<gi, kAdjBlock, 0, s>>>(a);
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
-    a.tau_base = gi;
-    lbm::adjoint_kernel<S, A, VB, lbm::ROWS_FACES, MACRO><<<gf, kAdjBlock, 0, s>>>(a);
-    return cudaGetLastError();
+    return macro ? lbm::launch_adjoint_kernel<S, A, true>(a, kAdjBlock, s)
+                 : lbm::launch_adjoint_kernel<S, A, false>(a, kAdjBlock, s);
 }
 template <class S>
 cudaError_t run_loss_seed(const lbm::AdjArgs &a, unsigned grid, cudaStream_t s)
@@ -119,10 +109,7 @@ cudaError_t run_lid_init_grad(const lbm::AdjArgs &a, cudaStream_t s)
 
 // ---- two steps per launch (FP32 adjoint)
 // z-planes per block (measured at 256^3: 16, 24, 32, 48 -> 24 best by 2%)
-#ifndef LBM_ADJ2_CHUNK
-#define LBM_ADJ2_CHUNK 24
-#endif
-constexpr int kAdj2Chunk = LBM_ADJ2_CHUNK;
+constexpr int kAdj2Chunk = 24;
 
 // blocks of the two-step launch (macro: the stored-point kernel's taller tiles)
 unsigned adj2_grid(const lbm_t *h, int &ntx, int &nty, bool macro)
@@ -136,14 +123,16 @@ unsigned adj2_grid(const lbm_t *h, int &ntx, int &nty, bool macro)
 }
 
 // Two steps per launch for the FP32 adjoint (adjoint_steps 0 or 2), up to
-// ADJ2_MAX_DIM.  By default only where its grid gives every SM two blocks or
-// more: a small lattice (64^3: 66 blocks) runs faster one step at a time.
+// ADJ2_MAX_DIM.  By default only on lattices where the second pass over the
+// adjoint that it saves is worth its ring of sites computed twice and its last
+// wave: backward us per iteration, stored points (FP16 storage; 96, 200 FP32),
+// one step / two: 64^3 7.2 / 12.3, 96^3 22.6 / 26.8, 128^3 51.4 / 53.2, 200^3
+// 193.4 / 192.8, 256^3 393 / 357; full states (with the recomputed forward)
+// 128^3 124 / 125, 256^3 912 / 870.
 bool two_step(const lbm_t *h)
 {
     if (adj64(h) || h->cfg.adjoint_steps == 1 || h->dim > lbm::ADJ2_MAX_DIM) return false;
-    if (h->cfg.adjoint_steps == 2) return true;
-    int ntx, nty;
-    return adj2_grid(h, ntx, nty, false) >= 2u * (unsigned)std::max(h->num_sms, 1);
+    return h->cfg.adjoint_steps == 2 || h->dim > 192;
 }
 
 template <class S, bool MACRO>
@@ -244,7 +233,6 @@ cudaError_t adjoint_two_steps(const lbm_t *h, const void *fwd_a, const void *fwd
     a.grad_lid = h->adj.grad_lid;
     a.tau_acc = h->adj.tau_acc;
     a.dim = h->dim;
-    a.zc = kAdj2Chunk;
     for (int i = 0; i < lbm::Q; ++i) {
         const long long sh = lbm::ex_of(i) + (long long)lbm::ey_of(i) * h->dim +
                              (long long)lbm::ez_of(i) * h->dim * h->dim;
@@ -253,6 +241,7 @@ cudaError_t adjoint_two_steps(const lbm_t *h, const void *fwd_a, const void *fwd
         a.off_down[i] = (unsigned)(base - (unsigned long long)sh);
         a.off_own[i] = (unsigned)base;
     }
+    a.zc = kAdj2Chunk;
     a.omega = (float)h->inv_tau;
     a.status = h->status;
     const unsigned grid = adj2_grid(h, a.ntx, a.nty, macro);
@@ -275,23 +264,14 @@ cudaError_t adjoint_two_steps(const lbm_t *h, const void *fwd_a, const void *fwd
     }
 }
 
-template <class S>
-cudaError_t run_adjoint_step_any(const lbm::AdjArgs &a, unsigned gi, unsigned gf, cudaStream_t s, bool macro)
-{
-    return macro ? run_adjoint_step<S, true>(a, gi, gf, s) : run_adjoint_step<S, false>(a, gi, gf, s);
-}
-
 cudaError_t adjoint_step(const lbm_t *h, const lbm::AdjArgs &a, bool macro)
 {
-    unsigned gi, gf;
-    adj_grids(h, gi, gf);
-    if (adj64(h) && h->prec != LBM_FP64)
-        return lbm::launch_adjoint_step_a64(h->prec, a, gi, gf, kAdjBlock, h->stream, macro);
+    if (adj64(h) && h->prec != LBM_FP64) return lbm::launch_adjoint_step_a64(h->prec, a, kAdjBlock, h->stream, macro);
     switch (h->prec) {
-    case LBM_FP32: return run_adjoint_step_any<float>(a, gi, gf, h->stream, macro);
-    case LBM_FP64: return run_adjoint_step_any<double>(a, gi, gf, h->stream, macro);
-    case LBM_FP16: return run_adjoint_step_any<__half>(a, gi, gf, h->stream, macro);
-    default: return run_adjoint_step_any<__nv_bfloat16>(a, gi, gf, h->stream, macro);
+    case LBM_FP32: return run_adjoint_step<float>(a, h->stream, macro);
+    case LBM_FP64: return run_adjoint_step<double>(a, h->stream, macro);
+    case LBM_FP16: return run_adjoint_step<__half>(a, h->stream, macro);
+    default: return run_adjoint_step<__nv_bfloat16>(a, h->stream, macro);
     }
 }
 
@@ -738,11 +718,9 @@ int lbm_adjoint_backward(lbm_t *h, double dloss, double *grad_tau, double *grad_
     if (grad_f0 && grad_f0_bytes != dbytes)
         return fail(LBM_EINVAL, "lbm_adjoint_backward: grad_f0 is %zu bytes, needs %zu", grad_f0_bytes, dbytes);
     const size_t nc = (size_t)h->dim * h->dim;
-    unsigned gi, gf;
-    adj_grids(h, gi, gf);
     int ntx, nty;
-    // tau partial slots: the one-step launch pair, or the two-step launch
-    const unsigned agrid = std::max(gi + gf, two_step(h) ? adj2_grid(h, ntx, nty, false) : 0u);
+    // tau partial slots: the one-step launch, or the two-step launch
+    const unsigned agrid = std::max(adj_grid(h), two_step(h) ? adj2_grid(h, ntx, nty, false) : 0u);
     if (!s.adj[0]) {
         int rc = alloc_tracked(h, &s.adj[0], abytes);
         if (rc == LBM_OK) rc = alloc_tracked(h, &s.adj[1], abytes);

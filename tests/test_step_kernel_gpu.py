@@ -35,3 +35,24 @@ def test_step_shapes_of_sizes_that_are_no_multiple_of_eight(capi, dim):
     for other in outs[1:]:
         for a, b in zip(outs[0], other):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp16", "bf16"])
+@pytest.mark.parametrize("dim,iters,every", [(8, 5, 2), (24, 9, 4), (104, 3, 3)])
+def test_one_step_adjoint_against_two_steps_per_launch(capi, prec, dim, iters, every):
+    """Gradients of the one-launch adjoint step (rows shorter and longer than
+    a block, both sweeps) against the two-step kernel's.  Tolerance: FP32
+    rounding of 19-term sums over the iterations, 1e-5 of the largest value."""
+    rng = np.random.default_rng(dim)
+    lid, target = 0.05 + 0.01 * rng.standard_normal(dim * dim), 0.02 * rng.standard_normal(dim * dim)
+    res = []
+    for steps in (1, 2):
+        for tau in (False, True):
+            with capi.Lattice(dim, velocity=0.0, precision=prec, lid=lid, tau=0.53, adjoint_steps=steps) as L:
+                L.adjoint_set_loss(dim // 2, target)
+                L.adjoint_forward(iters, every)
+                res.append(L.adjoint_backward(1.0, want_f0=False, want_tau=tau))
+    for one, two in zip(res[:2], res[2:]):
+        assert np.abs(one[1] - two[1]).max() <= 1e-5 * np.abs(two[1]).max()
+        if two[0] is not None:
+            assert abs(one[0] - two[0]) <= 1e-5 * abs(two[0])
