@@ -313,7 +313,7 @@ int alloc_tracked(lbm_t *h, void **p, size_t bytes)
     const size_t cap = h->cfg.max_device_bytes;
     if (cap > 0 && h->base_bytes + h->adj.bytes + bytes > cap)
         return fail(LBM_ENOMEM, "adjoint: needs %zu more device bytes, budget is %zu", bytes, cap);
-    ADJ_CUDA(cudaMalloc(p, bytes));
+    ADJ_CUDA(lbm::device_alloc(h, p, bytes));
     h->adj.bytes += bytes;
     return LBM_OK;
 }
@@ -324,6 +324,7 @@ size_t device_room(const lbm_t *h)
 {
     size_t freeb = 0, totalb = 0;
     if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) return 0;
+    freeb += lbm::device_cached(h);
     const size_t margin = ((size_t)1 << 30) + totalb / 50;
     size_t r = freeb > margin ? freeb - margin : 0;
     const size_t cap = h->cfg.max_device_bytes;
@@ -344,7 +345,7 @@ void drop_segment_graphs(lbm_adjoint_state &s)
 void free_tracked(lbm_t *h, void *p, size_t bytes)
 {
     if (!p) return;
-    cudaFree(p);
+    lbm::device_free(h, p);
     h->adj.bytes -= bytes;
 }
 
@@ -521,10 +522,10 @@ namespace lbm {
 void release_adjoint(lbm_t *h)
 {
     lbm_adjoint_state &s = h->adj;
-    for (void *p : s.ckpt) cudaFree(p);
-    for (void *p : s.seg) cudaFree(p);
-    for (void *p : s.mseg) cudaFree(p);
-    if (s.tail_block) cudaFree(s.tail_block);
+    for (void *p : s.ckpt) device_free(h, p);
+    for (void *p : s.seg) device_free(h, p);
+    for (void *p : s.mseg) device_free(h, p);
+    device_free(h, s.tail_block);
     s.tail_block = nullptr;
     s.tail_bytes = 0;
     s.ckpt.clear();
@@ -532,15 +533,15 @@ void release_adjoint(lbm_t *h)
     s.mseg.clear();
     s.tpts.clear();
     for (void *&p : s.mtmp) {
-        if (p) cudaFree(p);
+        device_free(h, p);
         p = nullptr;
     }
     for (void *&p : s.adj) {
-        if (p) cudaFree(p);
+        device_free(h, p);
         p = nullptr;
     }
     for (void *p : {(void *)s.grad_lid, (void *)s.tau_acc, (void *)s.loss_part, s.target, s.q0})
-        if (p) cudaFree(p);
+        device_free(h, p);
     s.q0 = nullptr;
     drop_segment_graphs(s);
     s.grad_lid = nullptr;

@@ -12,6 +12,8 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -134,7 +136,7 @@ void release(lbm_t *h)
     lbm::release_adjoint(h);
     for (void *p : {h->f[0], h->f[1], (void *)h->map, h->rho, h->u, h->lid, h->stage, (void *)h->partials,
                     (void *)h->red_out, (void *)h->status})
-        if (p) cudaFree(p);
+        lbm::device_free(h, p);
     for (auto &p : h->pending) {
         cudaEventDestroy(p.first);
         cudaEventDestroy(p.second);
@@ -142,6 +144,8 @@ void release(lbm_t *h)
     for (auto e : h->spare) cudaEventDestroy(e);
     for (cudaGraphExec_t &g : h->graph_exec)
         if (g) cudaGraphExecDestroy(g), g = nullptr;
+    // what the pool does not keep goes back now, not in some later call
+    if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->ev_first) cudaEventDestroy(h->ev_first);
     if (h->ev_last) cudaEventDestroy(h->ev_last);
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
@@ -149,6 +153,24 @@ void release(lbm_t *h)
     if (h->side) cudaStreamDestroy(h->side);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
+}
+
+// Name and SM count of a device, asked for once per process (0.2 ms a query).
+cudaError_t device_facts(int device, std::string &name, int &sms)
+{
+    static std::mutex mu;
+    static std::map<int, std::pair<std::string, int>> known;
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = known.find(device);
+    if (it == known.end()) {
+        cudaDeviceProp prop;
+        const cudaError_t e = cudaGetDeviceProperties(&prop, device);
+        if (e != cudaSuccess) return e;
+        it = known.emplace(device, std::make_pair(std::string(prop.name), prop.multiProcessorCount)).first;
+    }
+    name = it->second.first;
+    sms = it->second.second;
+    return cudaSuccess;
 }
 
 bool is_aa(const lbm_t *h) { return h->kernel == LBM_KERNEL_AA; }
@@ -544,28 +566,34 @@ int lbm_init(lbm_t **out, const lbm_config *c)
     int rc = LBM_OK;
     auto setup = [&]() -> int {
         LBM_CUDA(cudaSetDevice(c->device));
-        cudaDeviceProp prop;
-        LBM_CUDA(cudaGetDeviceProperties(&prop, c->device));
-        h->device_name = prop.name;
-        h->num_sms = prop.multiProcessorCount;
+        LBM_CUDA(device_facts(c->device, h->device_name, h->num_sms));
         h->graph_iters = c->graph_iterations == 0 ? 16 : c->graph_iterations;
         LBM_CUDA(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
-        LBM_CUDA(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
-        LBM_CUDA(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
-        LBM_CUDA(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
         LBM_CUDA(cudaEventCreate(&h->ev_first));
         LBM_CUDA(cudaEventCreate(&h->ev_last));
-        LBM_CUDA(cudaMalloc(&h->f[0], fbytes));
-        if (!aa) LBM_CUDA(cudaMalloc(&h->f[1], fbytes));
-        LBM_CUDA(cudaMalloc((void **)&h->map, n));
-        LBM_CUDA(cudaMalloc(&h->rho, n * mb));
-        LBM_CUDA(cudaMalloc(&h->u, 3 * n * mb));
-        LBM_CUDA(cudaMalloc(&h->lid, (size_t)dim * dim * mb));
-        LBM_CUDA(cudaMalloc(&h->stage, stage_elems * dump_elem(prec)));
-        LBM_CUDA(cudaMalloc((void **)&h->partials, (grid + 2) * 2 * sizeof(double)));
-        LBM_CUDA(cudaMalloc((void **)&h->red_out, 4 * sizeof(double)));
-        LBM_CUDA(cudaMalloc((void **)&h->status, sizeof(int)));
+        LBM_CUDA(lbm::device_alloc(h, &h->f[0], fbytes));
+        if (!aa) LBM_CUDA(lbm::device_alloc(h, &h->f[1], fbytes));
+        LBM_CUDA(lbm::device_alloc(h, (void **)&h->map, n));
+        LBM_CUDA(lbm::device_alloc(h, &h->rho, n * mb));
+        LBM_CUDA(lbm::device_alloc(h, &h->u, 3 * n * mb));
+        LBM_CUDA(lbm::device_alloc(h, &h->lid, (size_t)dim * dim * mb));
+        LBM_CUDA(lbm::device_alloc(h, &h->stage, stage_elems * dump_elem(prec)));
+        LBM_CUDA(lbm::device_alloc(h, (void **)&h->partials, (grid + 2) * 2 * sizeof(double)));
+        LBM_CUDA(lbm::device_alloc(h, (void **)&h->red_out, 4 * sizeof(double)));
+        LBM_CUDA(lbm::device_alloc(h, (void **)&h->status, sizeof(int)));
         LBM_CUDA(cudaMemsetAsync(h->status, 0, sizeof(int), h->stream));
+
+        // the wall rows of the second lattice: nothing writes them and no site
+        // uses them, but LBM_DUMP_F_RAW shows what reaches the walls' slots, and
+        // recycled memory would differ from run to run
+        if (!aa) {
+            const size_t row = (size_t)dim * sb, plane = row * dim, lattice = n * sb;
+            char *f1 = static_cast<char *>(h->f[1]);
+            for (size_t at : {(size_t)0, lattice - plane})
+                LBM_CUDA(cudaMemset2DAsync(f1 + at, lattice, 0, plane, lbm::Q, h->stream));
+            for (size_t at : {(size_t)0, plane - row})
+                LBM_CUDA(cudaMemset2DAsync(f1 + at, plane, 0, row, (size_t)lbm::Q * dim, h->stream));
+        }
 
         // lid profile in the macro precision (the reference's VELOCITY is a
         // literal of the kernel's real type, lbmcl.hpp:141)
@@ -608,6 +636,11 @@ int lbm_init(lbm_t **out, const lbm_config *c)
         // 32 threads 1539, 64 1527, 96 1556, 128 1558; FP32 200^3: 64 174.6,
         // 128 175.9, 256 183)
         h->step_block = c->block_threads > 0 ? block : 64u;
+        if (!h->step_vb) {
+            LBM_CUDA(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
+            LBM_CUDA(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
+            LBM_CUDA(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
+        }
         if (want == LBM_KERNEL_STAGED) {
             const int r = setup_staged(h, c->stages);
             if (r == LBM_OK) h->kernel = LBM_KERNEL_STAGED;

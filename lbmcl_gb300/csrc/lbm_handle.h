@@ -95,6 +95,8 @@ struct lbm_handle {
     // buffer parity and replayed (graph_iters = 1: no graphs)
     int graph_iters = 16;
     cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};
+    cudaMemPool_t pool = nullptr;  // where its device memory comes from (null: cudaMalloc)
+    bool pool_looked_up = false;
     bool state_is_init = true;  // the populations are what lbm_init made
     size_t base_bytes = 0;      // device bytes lbm_init allocated
     lbm_adjoint_state adj;
@@ -130,6 +132,11 @@ cudaError_t launch_iteration_adj(const lbm_t *h, const void *fin, void *fout, vo
 // h->graph_iters iterations from h->f[h->cur] as one replayed CUDA graph
 // (an even count: h->cur is unchanged)
 cudaError_t replay_iterations(lbm_t *h);
+// device memory of a handle, ordered on its stream (lbm_memory.cu); device_cached:
+// bytes its pool holds beside what is in use
+cudaError_t device_alloc(lbm_t *h, void **p, size_t bytes);
+void device_free(lbm_t *h, void *p);
+size_t device_cached(const lbm_t *h);
 // free the device memory of an adjoint state
 void release_adjoint(lbm_t *h);
 }  // namespace lbm

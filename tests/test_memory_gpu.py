@@ -1,0 +1,52 @@
+"""Handles share one device memory pool: handles made and destroyed in several
+threads at once, on recycled buffers, give the bits of a handle alone, and a
+gradient evaluated over and over keeps its value."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def run(capi, dim, prec, seed):
+    with capi.Lattice(dim, 0.005, 0.08, precision=prec, seed=seed, noise_sigma=1e-4) as L:
+        L.step(9, every=9)
+        return [a.view(np.uint8).copy() for a in (L.f(), L.rho(), L.u())] + [L.raw()]
+
+
+def test_threads_on_recycled_memory(capi):
+    jobs = [(24, "fp32", 1), (40, "fp16", 2), (32, "bf16", 3), (16, "fp64", 4)]
+    want = [run(capi, *j) for j in jobs]
+    bad = []
+
+    def work(k):
+        for r in range(6):
+            j = (k + r) % len(jobs)
+            for a, b in zip(run(capi, *jobs[j]), want[j]):
+                if not np.array_equal(a, b):
+                    bad.append((k, jobs[j]))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+
+
+@pytest.mark.parametrize("tau", [False, True])
+def test_gradients_on_recycled_memory(capi, tau):
+    got = []
+    for dim in (24, 40, 24, 32, 24):
+        lid = 0.05 + 0.01 * np.random.default_rng(dim).standard_normal(dim * dim)
+        with capi.Lattice(dim, velocity=0.0, precision="fp32", lid=lid, tau=0.53) as L:
+            L.adjoint_set_loss(dim // 2, None)
+            J = L.adjoint_forward(12, 5)
+            g = L.adjoint_backward(1.0, want_tau=tau)
+        if dim == 24:
+            got.append((J, g[0], g[1], g[2]))
+    for other in got[1:]:
+        assert got[0][0] == other[0] and got[0][1] == other[1]
+        np.testing.assert_array_equal(got[0][2], other[2])
+        np.testing.assert_array_equal(got[0][3], other[3])
