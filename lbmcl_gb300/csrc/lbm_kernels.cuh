@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "lbm_device.cuh"
+#include "lbm_fixed.cuh"
 #include "lbm_noise.cuh"
 
 
@@ -729,6 +730,26 @@ __device__ __forceinline__ void update_vector(S (&fs)[Q][V], typename MapWord<V>
 }
 
 
+// update_vector of one FP64 site of an interior row in 64-bit integers where
+// they serve (fx::fluid): the same bits.  False: not done, fs not valid.  The
+// row ends are not FLUID: nothing to do (face_fix, and walls nobody reads).
+template <int MODE>
+__device__ __forceinline__ bool update_fixed(double (&fs)[Q][1], const StepArgs &a, int x0, size_t site0)
+{
+    if ((unsigned)(x0 - 2) > (unsigned)(a.dim - 5)) return true;
+    if (a.sailfish) return false;
+    double f[Q];
+#pragma unroll
+    for (int i = 0; i < Q; ++i) f[i] = fs[i][0];
+    SiteOut o;
+    if (!fx::fluid(f, a.inv_tau, make_weights<double>(), o.r, o.ux, o.uy, o.uz)) return false;
+#pragma unroll
+    for (int i = 0; i < Q; ++i) fs[i][0] = f[i];
+    if (MODE == MODE_STEP_MACRO) store_macro<double>(a, site0, o);
+    if (MODE == MODE_STEP_ADJ) store_adj<double>(a, site0, o, false);
+    return true;
+}
+
 // Bounce-back of the x-face site x = xf of an interior row (y, z in
 // [2, dim-3]): its output population i is its pulled input of the opposite
 // direction, and an input whose source is the wall (x = 0 or dim-1) is the
@@ -770,7 +791,12 @@ __device__ __forceinline__ void pull_vector(const StepArgs &a, int xv, int y, in
     const S *__restrict__ fin = static_cast<const S *>(a.fin);
     S fs[Q][V];
     gather_all<S, V, 0, NC>(fin, a.n, rowoff, dim, x0, fs);
-    update_vector<S, MODE, V, INTERIOR>(fs, mw, a, y, z, x0, site0, red_m, red_e);
+    bool done = false;
+    if constexpr (std::is_same<S, double>::value && V == 1 && INTERIOR && MODE != MODE_REDUCE) {
+        done = update_fixed<MODE>(fs, a, x0, site0);
+        if (!done) gather_all<S, V, 0, NC>(fin, a.n, rowoff, dim, x0, fs);
+    }
+    if (!done) update_vector<S, MODE, V, INTERIOR>(fs, mw, a, y, z, x0, site0, red_m, red_e);
     if (INTERIOR && MODE != MODE_REDUCE) {
         // the walls (x = 0, dim-1) hold values nobody reads; the faces bounce back
         if constexpr (V == 1) {
@@ -825,12 +851,12 @@ __device__ __forceinline__ void decode_face_row(int dim, unsigned br, int &y, in
 // 65536 / (threads n).  Measured at 512^3 on GB300: 16-bit storage runs
 // fastest with 128 threads x 3 (168 registers: 84,448 MLUPS against 82,201 at
 // 128 registers, which spill 88 bytes); FP32 with 8-byte vectors at 85
-// registers (256 x 3); FP64 is FP64-throughput bound and left uncapped.
+// registers (256 x 3), FP64 with one site per thread at 128 (lbm_fixed.cuh).
 // lbm_init clamps block_threads to max_threads.
 template <class S> constexpr int max_threads() { return sizeof(S) == 2 ? 128 : 256; }
 template <class S, int VB> constexpr int min_blocks()
 {
-    return sizeof(S) == 2 ? (VB == 16 ? 3 : VB == 8 ? 4 : 6) : sizeof(S) == 4 ? (VB == 16 ? 2 : 3) : 1;
+    return sizeof(S) == 2 ? (VB == 16 ? 3 : VB == 8 ? 4 : 6) : sizeof(S) == 4 ? (VB == 16 ? 2 : 3) : (VB == 8 ? 2 : 1);
 }
 
 template <class S, int MODE, int VB, int ROWS>
@@ -874,15 +900,16 @@ __global__ void __launch_bounds__(max_threads<S>(), min_blocks<S, VB>()) pull_ke
 // visible) before they touch the lattices (0.1 - 0.3 us per iteration).
 // launch_dependents comes after the wait, so at most two iterations overlap.
 //
-// Face rows take two sites per thread whatever the interior's vectors: the
-// general update is long, short vectors keep its latency and registers down.
+// Face rows take two sites per thread whatever the interior's vectors (FP64
+// one: 16^3 13.9 -> 11.3 us): the general update is long, short vectors keep
+// its latency and registers down.
 // ---------------------------------------------------------------------------
-constexpr int FACE_VEC = 2;
+template <class S> __host__ __device__ constexpr int face_vec() { return sizeof(S) == 8 ? 1 : 2; }
 
 template <class S, int MODE, int VB>
 __global__ void __launch_bounds__(max_threads<S>(), min_blocks<S, VB>()) step_kernel(StepArgs a, StepRows r)
 {
-    constexpr int V = VB / (int)sizeof(S), VF = FACE_VEC;
+    constexpr int V = VB / (int)sizeof(S), VF = face_vec<S>();
     const int dim = a.dim;
     double red_m = 0.0, red_e = 0.0;  // unused
     if (blockIdx.x < r.face_blocks) {

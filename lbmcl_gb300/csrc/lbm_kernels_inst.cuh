@@ -108,7 +108,7 @@ cudaError_t LBM_CAT(launch_rows_, LBM_SFX)(int mode, const StepArgs &a, unsigned
 template <int VB, int MODE>
 static cudaError_t launch_step_mode(const StepArgs &a, unsigned block, cudaStream_t s)
 {
-    constexpr unsigned V = VB / (int)sizeof(LBM_S), VF = FACE_VEC;
+    constexpr unsigned V = VB / (int)sizeof(LBM_S), VF = face_vec<LBM_S>();
     const unsigned dim = (unsigned)a.dim, m = dim - 4;
     const size_t ni = (size_t)m * m * (dim / V), nf = (size_t)4 * (dim - 3) * (dim / VF);
     if (ni >> 31) return cudaErrorInvalidValue;  // FastDiv's range
