@@ -748,6 +748,9 @@ int lbm_dump(lbm_t *h, int what, void *dst, size_t bytes)
             a.sd = h->sd;
             a.n = h->n;
             a.layout = state_layout(h);
+            a.four = (h->sd < 0 || h->sd >= 2) && h->dim > 4 && h->n >> 29 == 0;
+            a.div_dim = lbm::FastDiv((unsigned)h->dim);
+            a.inv_n = ~0ull / h->n + 1;
             switch (h->prec) {
             case LBM_FP32: LBM_CUDA(lbm::launch_dump_f32(a, h->stream)); break;
             case LBM_FP64: LBM_CUDA(lbm::launch_dump_f64(a, h->stream)); break;
@@ -812,6 +815,9 @@ int lbm_load(lbm_t *h, int what, const void *src, size_t bytes)
             a.sd = h->sd;
             a.n = h->n;
             a.layout = state_layout(h);
+            a.four = (h->sd < 0 || h->sd >= 2) && h->dim > 4 && h->n >> 29 == 0;
+            a.div_dim = lbm::FastDiv((unsigned)h->dim);
+            a.inv_n = ~0ull / h->n + 1;
             LBM_CUDA(cudaMemcpyAsync(h->stage, (const char *)src + o0 * te, a.count * te, cudaMemcpyHostToDevice,
                                      h->stream));
             switch (h->prec) {

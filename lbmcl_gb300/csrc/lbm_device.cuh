@@ -423,6 +423,10 @@ struct DumpArgs {
     size_t n;
     int layout;           // LAYOUT_PULL: P of the two-lattice kernels; LAYOUT_AA_A / _B: the
                           // AA lattice in A-form / B-form
+    int four;             // 1: four elements are four sites of a row (stride >= 4 or SoA, dim > 4,
+                          // site numbers below 2^29)
+    FastDiv div_dim;      // by dim
+    unsigned long long inv_n;  // floor(2^64 / n) + 1: o inv_n / 2^64 floors to o / n for 19 n^2 < 2^64
 };
 enum { LAYOUT_PULL = -1, LAYOUT_AA_A = 0, LAYOUT_AA_B = 1 };
 

@@ -187,18 +187,20 @@ cudaError_t LBM_CAT(launch_init_, LBM_SFX)(const InitArgs &a, cudaStream_t s)
 cudaError_t LBM_CAT(launch_dump_, LBM_SFX)(const DumpArgs &a, cudaStream_t s)
 {
     const unsigned block = 256;
-    const size_t grid = (a.count + block - 1) / block;
+    const size_t grid = (a.count / (a.four ? 4 : 1) + block - 1) / block;  // a.count is a multiple of 4
     if (grid == 0) return cudaSuccess;
-    dump_f_kernel<LBM_S, LBM_T><<<(unsigned)grid, block, 0, s>>>(a);
+    if (a.four) dump_f_kernel<LBM_S, LBM_T><<<(unsigned)grid, block, 0, s>>>(a);
+    else dump_f_any_kernel<LBM_S, LBM_T><<<(unsigned)grid, block, 0, s>>>(a);
     return cudaGetLastError();
 }
 
 cudaError_t LBM_CAT(launch_load_, LBM_SFX)(const DumpArgs &a, cudaStream_t s)
 {
     const unsigned block = 256;
-    const size_t grid = (a.count + block - 1) / block;
+    const size_t grid = (a.count / (a.four ? 4 : 1) + block - 1) / block;  // a.count is a multiple of 4
     if (grid == 0) return cudaSuccess;
-    load_f_kernel<LBM_S, LBM_T><<<(unsigned)grid, block, 0, s>>>(a);
+    if (a.four) load_f_kernel<LBM_S, LBM_T><<<(unsigned)grid, block, 0, s>>>(a);
+    else load_f_any_kernel<LBM_S, LBM_T><<<(unsigned)grid, block, 0, s>>>(a);
     return cudaGetLastError();
 }
 

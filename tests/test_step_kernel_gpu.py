@@ -56,3 +56,28 @@ def test_one_step_adjoint_against_two_steps_per_launch(capi, prec, dim, iters, e
         assert np.abs(one[1] - two[1]).max() <= 1e-5 * np.abs(two[1]).max()
         if two[0] is not None:
             assert abs(one[0] - two[0]) <= 1e-5 * abs(two[0])
+
+
+@pytest.mark.parametrize("kernel,steps", [("auto", 3), ("aa", 3), ("aa", 4)])
+@pytest.mark.parametrize("prec,dim", [("fp32", 4), ("fp32", 12), ("fp64", 20), ("fp16", 24), ("bf16", 8)])
+def test_dump_and_load_agree_over_strides(capi, prec, dim, kernel, steps):
+    """The F dump of one state in every stride that divides dim^3 (elements one
+    by one and four at a time) re-indexed to SoA, and loading each into a
+    fresh handle gives that state back."""
+    want = None
+    strides = [0] + [1 << k for k in range(16) if dim ** 3 % (1 << k) == 0]
+    for st in strides:
+        with capi.Lattice(dim, 0.005, 0.08, precision=prec, seed=6, noise_sigma=1e-3, kernel=kernel,
+                          stride=st) as L:
+            L.step(steps)
+            f = L.f()
+            soa = f.reshape(19, -1) if st == 0 else f.reshape(-1, 19, st).transpose(1, 0, 2).reshape(19, -1)
+            soa = np.ascontiguousarray(soa)
+            want = soa if want is None else want
+            np.testing.assert_array_equal(soa.view(np.uint8), want.view(np.uint8))
+            L.step(2)
+            L.load_f(f)
+            # 16-bit storage rounds the dumped floats' deviations once more
+            got, tol = L.f(), (0 if prec in ("fp32", "fp64") else 1e-6)
+            assert np.array_equal(np.isnan(got), np.isnan(f))
+            assert np.nanmax(np.abs(got.astype(np.float64) - f)) <= tol
