@@ -115,7 +115,8 @@ typedef struct lbm_config {
                                   segment storing only the adjoint's linearisation point
                                   per iteration (u of FLUID sites, rho of lid sites: 3
                                   planes); 1 = store the full states, as with a tau
-                                  gradient                                                  */
+                                  gradient (and let the forward record states instead of
+                                  points, see adjoint_tail_segments)                        */
     int adjoint_fp64;          /* 1: the adjoint in FP64 arithmetic for FP32 / FP16 / BF16
                                   storage too (one step per launch), e.g. to measure the
                                   FP32 adjoint's rounding on the same trajectory; 0: FP64
@@ -136,7 +137,10 @@ typedef struct lbm_config {
                                   sweep without a tau gradient does not recompute them:
                                   0 = as many segments as fit in the device memory left
                                   beyond what the sweep itself needs, n > 0 = at most n,
-                                  -1 = none; the gradients are the same bit for bit       */
+                                  -1 = none; with adjoint_full_states it records the states
+                                  themselves (within a quarter of the device's memory), for
+                                  sweeps with or without a tau gradient; the gradients are
+                                  the same bit for bit                                     */
 } lbm_config;
 
 /* Iteration kernel variants (same results, different data movement). */

@@ -138,7 +138,8 @@ class Lattice:
     adjoint_tail_segments: checkpoint segments at the end of an adjoint
     forward whose linearisation points it records, so a backward sweep
     without a tau gradient skips recomputing them (0 = as many as fit, n = at
-    most n, -1 = none; same results).
+    most n, -1 = none; same results); with adjoint_full_states it records
+    their states, for sweeps with a tau gradient too.
     """
 
     def __init__(self, dim, viscosity=0.0089, velocity=0.05, precision="fp32", stride=None, lid=None,

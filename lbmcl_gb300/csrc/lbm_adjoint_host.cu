@@ -620,24 +620,43 @@ int lbm_adjoint_forward(lbm_t *h, int iterations, int checkpoint_every, double *
     s.every = c;
     s.init_state = h->state_is_init;
 
-    // The last mt segments record their linearisation points here (the
-    // stored-point backward sweep then skips recomputing them): as many as
-    // fit in the device memory left once the sweep's own buffers (c point
-    // sets, two state scratch buffers, the staged checkpoint, the two adjoint
-    // buffers) are set aside.
-    const size_t mbytes = 3 * h->n * lbm::macro_bytes(h->prec);
+    // The last mt segments record here what the backward sweep needs of each of
+    // their iterations, which then is not recomputed: the linearisation point,
+    // or with adjoint_full_states the state itself (each iteration's output goes
+    // to a buffer of its own).  As many as fit in the device memory left once
+    // the sweep's own buffers (the checkpoints above, a segment's point sets or
+    // states, two state scratch buffers, the staged checkpoint, the two adjoint
+    // buffers) are set aside.  States: within the quarter of the device's memory
+    // that the pool keeps from one handle to the next; mapping and unmapping one
+    // beyond it takes longer than the iteration it saves (256^3 FP16: 0.64 GB,
+    // 0.5 ms, against 0.21 ms).
+    const bool states = h->cfg.adjoint_full_states != 0;
+    const size_t mbytes = states ? fbytes : 3 * h->n * lbm::macro_bytes(h->prec);
     int mt = 0;
     if (h->cfg.adjoint_tail_segments >= 0) {
         const size_t abytes = (size_t)lbm::Q * h->n * adj_bytes(h);
         size_t reserve = ((size_t)1 << 30);
-        if (s.mseg.size() < (size_t)c) reserve += ((size_t)c - s.mseg.size()) * mbytes;
-        if (!s.mtmp[0]) reserve += 2 * fbytes;
+        if (states) reserve += (size_t)(c - 1) * fbytes;
+        else if (s.mseg.size() < (size_t)c) reserve += ((size_t)c - s.mseg.size()) * mbytes;
+        if (!states && !s.mtmp[0]) reserve += 2 * fbytes;
         if (!s.q0) reserve += fbytes;
-        if (!s.adj[0]) reserve += 2 * abytes + (size_t)h->dim * h->dim * sizeof(double);
-        const size_t r = device_room(h);
-        if (r > reserve) mt = (int)std::min<size_t>((size_t)nck, (r - reserve) / ((size_t)c * mbytes));
+        const size_t sweep = s.adj[0] ? (size_t)0 : 2 * abytes + (size_t)h->dim * h->dim * sizeof(double);
+        reserve += sweep;
+        size_t r = device_room(h);
+        if (states) {
+            size_t freeb = 0, totalb = 0;
+            if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) totalb = 0;
+            const size_t used = h->base_bytes + s.bytes;
+            r = std::min(r, totalb / 4 > used ? totalb / 4 - used : (size_t)0);
+        }
+        // with every segment recorded nothing of a segment's recompute is held
+        const size_t whole = (size_t)iterations * mbytes + ((size_t)1 << 30) + sweep;
+        if (states && h->cfg.adjoint_max_states > 0) mt = 0;  // the caller limits state buffers
+        else if (states && r >= whole) mt = nck;
+        else if (r > reserve) mt = (int)std::min<size_t>((size_t)nck, (r - reserve) / ((size_t)c * mbytes));
         if (h->cfg.adjoint_tail_segments > 0) mt = std::min(mt, h->cfg.adjoint_tail_segments);
     }
+    s.tail_states = states;
     s.tail_k0 = (nck - mt) * c;
     if (s.tail_k0 < iterations) {
         const size_t bytes = (size_t)(iterations - s.tail_k0) * mbytes;
@@ -656,11 +675,20 @@ int lbm_adjoint_forward(lbm_t *h, int iterations, int checkpoint_every, double *
 
     // Q_0, then the iterations, copying Q_{jc} into checkpoint j; runs that
     // stay inside one checkpoint interval replay the step graph; the tail's
-    // iterations also store their points
+    // iterations also store their points, or leave their input where it is
+    // (recorded states: iteration k reads tpts[k - tail_k0] and writes the next
+    // one, the last one a lattice buffer)
     ADJ_CUDA(cudaMemcpyAsync(s.ckpt[0], h->f[h->cur], fbytes, cudaMemcpyDeviceToDevice, h->stream));
     for (int k = 0; k < iterations;) {
         const int G = h->graph_iters, next_ck = (k / c + 1) * c;
-        if (k >= s.tail_k0) {
+        if (k >= s.tail_k0 && states) {
+            if (k == s.tail_k0)
+                ADJ_CUDA(cudaMemcpyAsync(s.tpts[0], h->f[h->cur], fbytes, cudaMemcpyDeviceToDevice, h->stream));
+            const size_t at = (size_t)(k - s.tail_k0);
+            ADJ_CUDA(lbm::launch_iteration(h, s.tpts[at], k + 1 < iterations ? s.tpts[at + 1] : h->f[h->cur]));
+            ++k;
+            continue;
+        } else if (k >= s.tail_k0) {
             ADJ_CUDA(lbm::launch_iteration_adj(h, h->f[h->cur], h->f[h->cur ^ 1], s.tpts[k - s.tail_k0]));
             h->cur ^= 1;
             ++k;
@@ -765,8 +793,10 @@ int lbm_adjoint_backward(lbm_t *h, double dloss, double *grad_tau, double *grad_
     // are recomputed storing those three planes (c of them, plus two state
     // scratch buffers) instead of c - 1 full states.
     bool macro = grad_tau == nullptr && !h->cfg.adjoint_full_states;
-    // the recorded tail points serve the stored-point sweep only
-    if (!macro) free_tail_points(h);
+    // recorded points serve the stored-point sweep only (and recorded states,
+    // with adjoint_full_states, the full-state sweep only)
+    if (macro == s.tail_states) free_tail_points(h);
+    const bool all_states = s.tail_states && s.tail_k0 == 0;  // nothing to recompute
     if (macro) {
         // the full-state buffers of an earlier sweep make room first (and
         // the graphs that captured them go)
@@ -806,7 +836,7 @@ int lbm_adjoint_backward(lbm_t *h, double dloss, double *grad_tau, double *grad_
     // checkpointing), else as many as fit, and the sweep recurses.  Allocated
     // on the first backward sweep only, so a loss-only forward holds just its
     // checkpoints.
-    if (!macro && (int)s.seg.size() < c - 1) {
+    if (!macro && !all_states && (int)s.seg.size() < c - 1) {
         size_t fit = room() / fbytes;
         size_t want_total = (size_t)(c - 1);
         if (h->cfg.adjoint_max_states > 0) want_total = std::min(want_total, (size_t)h->cfg.adjoint_max_states);
@@ -831,7 +861,7 @@ int lbm_adjoint_backward(lbm_t *h, double dloss, double *grad_tau, double *grad_
     // per segment) when graphs are on and the copy buffer fits.
     ADJ_CUDA(prepare_adjoint2(h));
     const int nck = (T + c - 1) / c;
-    bool graphs = h->graph_iters > 1 && c >= 2 && (macro || (int)s.seg.size() >= c - 1);
+    bool graphs = h->graph_iters > 1 && c >= 2 && !all_states && (macro || (int)s.seg.size() >= c - 1);
     if (graphs && (s.seg_graph_c != c || s.seg_graph_macro != macro)) {  // graphs of another sweep
         drop_segment_graphs(s);
         s.seg_graph_c = c;
@@ -842,10 +872,10 @@ int lbm_adjoint_backward(lbm_t *h, double dloss, double *grad_tau, double *grad_
     }
     for (int j = nck - 1; j >= 0; --j) {
         const int start = j * c, len = std::min(T, start + c) - start;
-        if (macro && start >= s.tail_k0) {
-            // points recorded by the forward: the adjoint steps only
+        if (start >= s.tail_k0) {
+            // points or states recorded by the forward: the adjoint steps only
             const int rc = adjoint_steps_down(h, start, len,
-                                              [&](int k) -> const void * { return s.tpts[k - s.tail_k0]; }, cur, true);
+                                              [&](int k) -> const void * { return s.tpts[k - s.tail_k0]; }, cur, macro);
             if (rc != LBM_OK) return rc;
             continue;
         }

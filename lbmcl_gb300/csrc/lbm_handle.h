@@ -39,9 +39,10 @@ struct lbm_adjoint_state {
     // iteration of one segment (3 planes each) and two state scratch buffers
     std::vector<void *> mseg;
     void *mtmp[2] = {nullptr, nullptr};
-    // the points of the iterations tail_k0 .. T-1 (the last segments),
-    // recorded by the adjoint forward into one allocation: those segments
-    // are not recomputed
+    // the points (or, tail_states, the states they start from) of the
+    // iterations tail_k0 .. T-1 (the last segments), recorded by the adjoint
+    // forward into one allocation: those segments are not recomputed
+    bool tail_states = false;
     void *tail_block = nullptr;
     size_t tail_bytes = 0;
     std::vector<void *> tpts;  // per iteration, into tail_block

@@ -50,3 +50,31 @@ def test_gradients_on_recycled_memory(capi, tau):
         assert got[0][0] == other[0] and got[0][1] == other[1]
         np.testing.assert_array_equal(got[0][2], other[2])
         np.testing.assert_array_equal(got[0][3], other[3])
+
+
+@pytest.mark.parametrize("prec,steps", [("fp32", 2), ("fp16", 1), ("bf16", 2), ("fp64", 1)])
+@pytest.mark.parametrize("dim,iters,every", [(24, 37, 8), (40, 20, 10), (16, 5, 7)])
+def test_recorded_states_are_exact(capi, prec, steps, dim, iters, every):
+    """With adjoint_full_states the forward records the states of its last
+    segments (all, two, one): the loss, the state it ends in and the gradients
+    of sweeps with and without a tau gradient are those of recomputing."""
+    rng = np.random.default_rng(dim + iters)
+    lid, target = 0.05 + 0.01 * rng.standard_normal(dim * dim), 0.02 * rng.standard_normal(dim * dim)
+    res = []
+    for tail in (-1, 0, 2, 1):
+        for tau in (True, False):
+            with capi.Lattice(dim, velocity=0.0, precision=prec, lid=lid, tau=0.53, seed=3, noise_sigma=1e-4,
+                              adjoint_steps=steps, adjoint_full_states=True, adjoint_tail_segments=tail) as L:
+                L.adjoint_set_loss(dim // 2, target)
+                out = []
+                for _ in range(2):  # the second run starts from the first one's end
+                    J = L.adjoint_forward(iters, every)
+                    out.append((J, L.f()) + tuple(L.adjoint_backward(1.0, want_tau=tau)))
+            res.append(out)
+    for k in (2, 4, 6):
+        for tau in (0, 1):
+            for a, b in zip(res[tau], res[k + tau]):
+                assert a[0] == b[0] and a[2] == b[2]
+                np.testing.assert_array_equal(a[1], b[1])
+                np.testing.assert_array_equal(a[3], b[3])
+                np.testing.assert_array_equal(a[4], b[4])
