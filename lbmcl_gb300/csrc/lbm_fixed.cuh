@@ -28,8 +28,7 @@
 // |u_x|, |u_y|, |u_z| < 1/8, rho in [7/8, 2), feq - f a double, as it is within a
 // factor of two, |feq - f| / tau < 1/2, 2^-10 <= 1/tau < 64) hold for
 // flows well inside the low-Mach range of the scheme; a site outside any of
-// them, or with the one divisor the reciprocal may round wrongly for, reports
-// false and takes the IEEE path.
+// them reports false and takes the IEEE path.
 #pragma once
 
 #include "lbm_device.cuh"
@@ -116,16 +115,16 @@ struct Extremes {
 
 // Correctly rounded x / r, y / r, z / r for r in [2^-4, 8), |x|, |y|, |z| zero
 // or in [2^-64, 8), from one reciprocal: a single-precision seed, three Newton
-// steps, then q = x y and q + (x - r q) y with exact remainders.  After the
-// third step y is the reciprocal correctly rounded, whatever r but the one
-// whose mantissa is all ones, and the corrected quotient then is the correctly
-// rounded one (P. W. Markstein, "Computation of elementary functions on the IBM
-// RISC System/6000 processor", IBM J. Res. Develop. 34 (1990)).  False for that
-// r.  15 FP64 operations; three IEEE divisions take about 42.
-__device__ __forceinline__ bool divide3(double x, double y, double z, double r, double &qx, double &qy, double &qz)
+// steps, then q = x c and q + (x - r q) c with exact remainders.  After the
+// third step c is the reciprocal correctly rounded, unless r's mantissa is all
+// ones (its reciprocal lies an ulp above the power of two the step returns),
+// and the corrected quotient then is the correctly rounded one (P. W.
+// Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Develop. 34 (1990)).  15 FP64 operations; three IEEE
+// divisions take about 42.
+__device__ __forceinline__ void quotients(double x, double y, double z, double r, double &qx, double &qy, double &qz)
 {
     const u64 b = bits(r);
-    if ((lo32(b) == 0xffffffffu) && ((hi32(b) & 0xfffffu) == 0xfffffu)) return false;
     // r truncated to single precision and the seed back to double: both exact
     // in the exponent range of r, as integer operations
     const unsigned fb = ((hi32(b) - (896u << 20)) << 3) | (lo32(b) >> 29);
@@ -133,12 +132,12 @@ __device__ __forceinline__ bool divide3(double x, double y, double z, double r, 
     double c = value(make64((gb >> 3) + (896u << 20), gb << 29));
     c = __fma_rn(c, __fma_rn(-r, c, 1.0), c);  // 2^-22 -> 2^-44
     c = __fma_rn(c, __fma_rn(-r, c, 1.0), c);  // within an ulp
-    c = __fma_rn(c, __fma_rn(-r, c, 1.0), c);  // correctly rounded
+    c = __fma_rn(c, __fma_rn(-r, c, 1.0), c);  // correctly rounded, unless r's mantissa is all ones
+    if (lo32(b) == 0xffffffffu && (hi32(b) & 0xfffffu) == 0xfffffu) c = value(make64((2045u - (hi32(b) >> 20)) << 20, 1));
     const double px = __dmul_rn(x, c), py = __dmul_rn(y, c), pz = __dmul_rn(z, c);
     qx = __fma_rn(__fma_rn(-r, px, x), c, px);
     qy = __fma_rn(__fma_rn(-r, py, y), c, py);
     qz = __fma_rn(__fma_rn(-r, pz, z), c, pz);
-    return true;
 }
 
 // f + inv_tau (feq - f), f as F in fixed point, feq in [2^-8, 4)
@@ -192,7 +191,7 @@ __device__ __forceinline__ bool fluid(double (&f)[Q], double inv_tau, const Weig
     const double pz = to_double(round53(round53(round53(F[6] + F[15]) + F[16]) + F[17]) + F[18]);
     const double mz = to_double(round53(round53(round53(F[5] + F[11]) + F[12]) + F[13]) + F[14]);
     double ux, uy, uz;
-    if (!divide3(__dsub_rn(px, mx), __dsub_rn(py, my), __dsub_rn(pz, mz), r, ux, uy, uz)) return false;
+    quotients(__dsub_rn(px, mx), __dsub_rn(py, my), __dsub_rn(pz, mz), r, ux, uy, uz);
     const unsigned top = 1020u << 20;  // 1/8
     // rho in [7/8, 2): with |u_i| < 1/8 every bracket is at least 0.46 and
     // every feq at least 0.011
