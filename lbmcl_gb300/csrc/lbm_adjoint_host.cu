@@ -707,7 +707,7 @@ int lbm_adjoint_forward(lbm_t *h, int iterations, int checkpoint_every, double *
     h->state_is_init = false;
 
     // loss of R_T = S(Q_T)
-    s.loss_grid = (unsigned)((h->n + kLossBlock - 1) / kLossBlock);
+    s.loss_grid = (unsigned)(((size_t)h->dim * h->dim + kLossBlock - 1) / kLossBlock);
     if (!s.loss_part) {
         int rc = alloc_tracked(h, (void **)&s.loss_part, ((size_t)s.loss_grid + 1) * 2 * sizeof(double));
         if (rc != LBM_OK) return rc;
