@@ -331,12 +331,18 @@ cudaError_t launch_pull(const lbm_t *h, int mode, const lbm::StepArgs &a, unsign
         default: return lbm::launch_staged_bf16(mode, a, h->sgrid, h->sblock, h->ssmem, h->stream);
         }
     }
-    if (!h->step_vb) return launch_rows(h, mode, a, h->stream);
+    // Iterations that also store the linearisation points need registers for
+    // them: 16-bit storage with 8-byte vectors at every size beyond 40^3 (us per
+    // iteration of the adjoint forward, 16-byte vectors -> 8: FP16 96^3 15.1 ->
+    // 14.5, 256^3 262 -> 250; BF16 128^3 38.6 -> 36.5, 256^3 278 -> 253).
+    const bool s16 = h->prec == LBM_FP16 || h->prec == LBM_BF16;
+    const int vb = mode == lbm::MODE_STEP_ADJ && s16 && h->step_vb != 4 ? 8 : h->step_vb;
+    if (!vb) return launch_rows(h, mode, a, h->stream);
     switch (h->prec) {
-    case LBM_FP32: return lbm::launch_step_f32(h->step_vb, mode, a, h->step_block, h->stream);
-    case LBM_FP64: return lbm::launch_step_f64(h->step_vb, mode, a, h->step_block, h->stream);
-    case LBM_FP16: return lbm::launch_step_f16(h->step_vb, mode, a, h->step_block, h->stream);
-    default: return lbm::launch_step_bf16(h->step_vb, mode, a, h->step_block, h->stream);
+    case LBM_FP32: return lbm::launch_step_f32(vb, mode, a, h->step_block, h->stream);
+    case LBM_FP64: return lbm::launch_step_f64(vb, mode, a, h->step_block, h->stream);
+    case LBM_FP16: return lbm::launch_step_f16(vb, mode, a, h->step_block, h->stream);
+    default: return lbm::launch_step_bf16(vb, mode, a, h->step_block, h->stream);
     }
 }
 
@@ -353,17 +359,16 @@ bool macro_within(int64_t it0, int G, int macro_every)
 // the two-launch iterations
 bool splits(const lbm_t *h) { return h->kernel != LBM_KERNEL_AA && h->kernel != LBM_KERNEL_STAGED && !h->step_vb; }
 
-// One two-launch iteration (MODE_STEP or MODE_STEP_ADJ) with its face-row
-// launch on the side stream, forked from and joined back into the handle's
+// One two-launch iteration with its face-row launch on the side stream, forked from and joined back into the handle's
 // stream, so that (in a captured graph: as a second branch) it runs beside the
 // interior-row launch; the two write disjoint rows of the output and read the
 // same input.
-cudaError_t split_iteration(const lbm_t *h, int mode, const lbm::StepArgs &a)
+cudaError_t split_iteration(const lbm_t *h, const lbm::StepArgs &a)
 {
     cudaError_t e = cudaEventRecord(h->ev_fork, h->stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->ev_fork, 0);
     if (e != cudaSuccess) return e;
-    e = launch_rows(h, mode, a, h->side);
+    e = launch_rows(h, lbm::MODE_STEP, a, h->side);
     // join even after a failed launch, so the capture can end
     const cudaError_t ej = cudaEventRecord(h->ev_join, h->side);
     const cudaError_t ew = ej == cudaSuccess ? cudaStreamWaitEvent(h->stream, h->ev_join, 0) : ej;
@@ -384,7 +389,7 @@ cudaError_t replay_graph(lbm_t *h)
         if (e != cudaSuccess) return e;
         int cur = h->cur, ph = h->aa_phase;
         for (int k = 0; k < h->graph_iters && e == cudaSuccess; ++k) {
-            e = split ? split_iteration(h, lbm::MODE_STEP, step_args(h, cur, ph))
+            e = split ? split_iteration(h, step_args(h, cur, ph))
                       : launch_pull(h, lbm::MODE_STEP, step_args(h, cur, ph));
             if (is_aa(h)) ph ^= 1;
             else cur ^= 1;
@@ -412,7 +417,7 @@ cudaError_t launch_iteration(const lbm_t *h, const void *fin, void *fout)
     StepArgs a = step_args(h, h->cur);
     a.fin = fin;
     a.fout = fout;
-    return splits(h) ? split_iteration(h, MODE_STEP, a) : launch_pull(h, MODE_STEP, a);
+    return splits(h) ? split_iteration(h, a) : launch_pull(h, MODE_STEP, a);
 }
 
 cudaError_t launch_iteration_adj(const lbm_t *h, const void *fin, void *fout, void *point)
@@ -422,7 +427,7 @@ cudaError_t launch_iteration_adj(const lbm_t *h, const void *fin, void *fout, vo
     a.fout = fout;
     a.rho = nullptr;
     a.u = point;
-    return splits(h) ? split_iteration(h, MODE_STEP_ADJ, a) : launch_pull(h, MODE_STEP_ADJ, a);
+    return launch_pull(h, MODE_STEP_ADJ, a);
 }
 }  // namespace lbm
 

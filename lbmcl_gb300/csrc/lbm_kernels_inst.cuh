@@ -97,7 +97,6 @@ cudaError_t LBM_CAT(launch_rows_, LBM_SFX)(int mode, const StepArgs &a, unsigned
         switch (mode) {
         case MODE_STEP: return launch_rows_mode<MODE_STEP>(a, block, s, sf, nullptr);
         case MODE_STEP_MACRO: return launch_rows_mode<MODE_STEP_MACRO>(a, block, s, sf, nullptr);
-        case MODE_STEP_ADJ: return launch_rows_mode<MODE_STEP_ADJ>(a, block, s, sf, nullptr);
         }
     }
     return cudaErrorInvalidValue;
