@@ -275,12 +275,15 @@ int setup_staged(lbm_t *h, int want_stages)
 // one or two sites per thread (its time is the latency of one thread's work
 // after a launch), a large one the fewest instructions.  us per iteration in
 // replayed graphs, 4- / 8- / 16-byte vectors, one launch; two launches:
-//   FP16  32^3  2.3 / 2.8 / 4.1; 4.9   64^3 5.8 / 5.1 / 6.7; 6.0
-//         96^3 14.1 / 11.9 / 11.8; 12.4   128^3 34.2 / 31.3 / 29.1; 30.0
-//         200^3  122 / 111 / 104.7; 103.5   256^3  253 / 211 / 208; 203
-//         512^3 1897 / 1648 / 1610; 1527
-//   BF16  32^3  2.3 / 2.6 / 3.6; 6.0   64^3 5.6 / 5.0 / 6.5; 7.0
-//         128^3 31.6 / 29.1 / 28.6; 31.4   200^3 105.5; 106.3   256^3 208; 205
+//   FP16  32^3  2.4 / 2.4 / 4.1; 4.9   64^3 5.6 / 5.0 / 6.7; 6.0
+//         96^3 14.0 / 10.9 / 11.8; 12.4   112^3 - / 19.6 / 18.8
+//         128^3 34 / 28.9 / 29.0; 30.0   160^3 - / 54.4 / 55.0; 56.3
+//         200^3 - / 104.7 / 104.7; 103.3   256^3 - / 199 / 208; 203
+//         320^3 - / 398 / -; 389   512^3 - / 1604 / 1610; 1527
+//   BF16  32^3  2.4 / 2.4 / 3.6; 6.0   64^3 5.6 / 5.0 / 6.5; 7.0
+//         96^3 13 / 11.4 / 11.6; 13.8   112^3 - / 19.8 / 18.5
+//         128^3 31.6 / 29.2 / 28.8; 31.4   200^3 - / 105.8 / 105.5; 106.2
+//         256^3 - / 201 / 208; 206   512^3 - / 1619 / 1597; 1560
 //   FP32  32^3  2.9 / 3.2 / 4.9; 3.8   64^3 8.1 / 7.5 / 9.0; 7.9
 //         128^3 57 / 48.0 / 55; 50.7   256^3 400 / 360 / 415; 375
 //         512^3 3157 / 2910 / 3217; 2950
@@ -295,7 +298,7 @@ int step_shape(int kernel, int prec, int dim)
     if (prec == LBM_FP32) return dim <= 40 ? 4 : 8;
     if (dim > 192) return 0;
     if (kernel == LBM_KERNEL_DIRECT) return 16;
-    return dim <= 40 ? 4 : dim <= 72 ? 8 : 16;
+    return dim <= 40 ? 4 : dim <= 104 ? 8 : 16;
 }
 
 // The two launches of an iteration with 16-byte vectors, face rows on sf.

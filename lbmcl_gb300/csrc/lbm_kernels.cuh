@@ -342,9 +342,7 @@ __device__ __forceinline__ void fluid_dev(float (&D)[Q], const DevK &K, SiteOut 
 // Two FLUID sites at once on packed FP32 pairs (lane .x one site, .y the
 // other): the operations of moments_dev / fluid_dev in the same order and
 // rounding (add/mul/fma .rn on f32x2), so each lane's result is bit for bit
-// the scalar one, in fewer arithmetic instructions.  RELAX2: the BGK update
-// packed too (its constants then live as register pairs), else per lane with
-// the scalar relax_pair_dev.
+// the scalar one, in fewer arithmetic instructions.
 __device__ __forceinline__ float2 f2_(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
@@ -362,7 +360,7 @@ __device__ __forceinline__ void relax_pair_dev2(float2 &dp, float2 &dm, float2 a
     dm = fma2(f2_(K.keep), dm, fma2(f2_(K.k[c]), X, neg2(lin)));
 }
 
-template <bool COLLIDE, bool RELAX2>
+template <bool COLLIDE>
 __device__ __forceinline__ void fluid_dev2(float2 (&D)[Q], const DevK &K, SiteOut &o0, SiteOut &o1)
 {
     const float2 s13 = add2(D[1], D[3]), d13 = sub2(D[1], D[3]);
@@ -389,31 +387,17 @@ __device__ __forceinline__ void fluid_dev2(float2 (&D)[Q], const DevK &K, SiteOu
     o0.r = rho.x; o0.ux = ux.x; o0.uy = uy.x; o0.uz = uz.x;
     o1.r = rho.y; o1.ux = ux.y; o1.uy = uy.y; o1.uz = uz.y;
     if (!COLLIDE) return;
-    if constexpr (RELAX2) {
-        const float2 c15 = mul2(f2_(1.5f), fma2(ux, ux, fma2(uy, uy, mul2(uz, uz))));
-        D[0] = fma2(f2_(K.keep), D[0], mul2(f2_(K.k[0]), fma2(rho, neg2(c15), drho)));
-        relax_pair_dev2(D[1], D[3], ux, 1, rho, drho, c15, K);
-        relax_pair_dev2(D[2], D[4], uy, 1, rho, drho, c15, K);
-        relax_pair_dev2(D[6], D[5], uz, 1, rho, drho, c15, K);
-        relax_pair_dev2(D[7], D[9], add2(ux, uy), 2, rho, drho, c15, K);
-        relax_pair_dev2(D[8], D[10], sub2(uy, ux), 2, rho, drho, c15, K);
-        relax_pair_dev2(D[11], D[17], sub2(ux, uz), 2, rho, drho, c15, K);
-        relax_pair_dev2(D[12], D[18], sub2(uy, uz), 2, rho, drho, c15, K);
-        relax_pair_dev2(D[15], D[13], add2(ux, uz), 2, rho, drho, c15, K);
-        relax_pair_dev2(D[16], D[14], add2(uy, uz), 2, rho, drho, c15, K);
-    } else {
-        float L[Q];
-#pragma unroll
-        for (int i = 0; i < Q; ++i) L[i] = D[i].x;
-        relax_dev(L, drho.x, rho.x, ux.x, uy.x, uz.x, K);
-#pragma unroll
-        for (int i = 0; i < Q; ++i) D[i].x = L[i];
-#pragma unroll
-        for (int i = 0; i < Q; ++i) L[i] = D[i].y;
-        relax_dev(L, drho.y, rho.y, ux.y, uy.y, uz.y, K);
-#pragma unroll
-        for (int i = 0; i < Q; ++i) D[i].y = L[i];
-    }
+    const float2 c15 = mul2(f2_(1.5f), fma2(ux, ux, fma2(uy, uy, mul2(uz, uz))));
+    D[0] = fma2(f2_(K.keep), D[0], mul2(f2_(K.k[0]), fma2(rho, neg2(c15), drho)));
+    relax_pair_dev2(D[1], D[3], ux, 1, rho, drho, c15, K);
+    relax_pair_dev2(D[2], D[4], uy, 1, rho, drho, c15, K);
+    relax_pair_dev2(D[6], D[5], uz, 1, rho, drho, c15, K);
+    relax_pair_dev2(D[7], D[9], add2(ux, uy), 2, rho, drho, c15, K);
+    relax_pair_dev2(D[8], D[10], sub2(uy, ux), 2, rho, drho, c15, K);
+    relax_pair_dev2(D[11], D[17], sub2(ux, uz), 2, rho, drho, c15, K);
+    relax_pair_dev2(D[12], D[18], sub2(uy, uz), 2, rho, drho, c15, K);
+    relax_pair_dev2(D[15], D[13], add2(ux, uz), 2, rho, drho, c15, K);
+    relax_pair_dev2(D[16], D[14], add2(uy, uz), 2, rho, drho, c15, K);
 }
 
 // Any site in deviation form (walls, faces, corners, lid, fluid).
@@ -620,19 +604,14 @@ __device__ __forceinline__ void update_general(S (&fs)[Q][V], typename MapWord<V
 }
 
 // Instruction form of the all-FLUID pairs of the 16-bit kernels (the same
-// bits either way): 0 = two scalar site updates, 1 = packed FP32x2 moments
-// and scalar BGK updates, 2 = packed throughout.  Chosen per storage type by
-// measurement at 512^3 (the packed forms change the register allocation at
-// the 168-register cap, which decides).
-#ifndef LBM_DEV16_FORM_F16
-#define LBM_DEV16_FORM_F16 0
-#endif
-#ifndef LBM_DEV16_FORM_BF16
-#define LBM_DEV16_FORM_BF16 2
-#endif
-template <class S> __host__ __device__ constexpr int dev16_form()
+// bits either way): 0 = two scalar site updates, 2 = packed FP32x2.  Packed is
+// a fifth fewer instructions; FP16 with eight sites per thread spills 80 bytes
+// that way at the 168-register cap and is scalar there (512^3 84,999 MLUPS
+// against 81,241; with four sites per thread, no spills, packed: 96^3 12.0 ->
+// 10.9 us, 256^3 211 -> 200).
+template <class S, int V> __host__ __device__ constexpr int dev16_form()
 {
-    return sizeof(S) != 2 ? 0 : (std::is_same<S, __half>::value ? LBM_DEV16_FORM_F16 : LBM_DEV16_FORM_BF16);
+    return sizeof(S) != 2 || (std::is_same<S, __half>::value && V == 8) ? 0 : 2;
 }
 
 // Update the V sites x0..x0+V-1 of row (y, z) in place: fs holds their pulled
@@ -687,7 +666,7 @@ __device__ __forceinline__ void update_vector(S (&fs)[Q][V], typename MapWord<V>
 #pragma unroll
             for (int k = 0; k < V; k += 2) {
                 SiteOut o0, o1;
-                if constexpr (dev16_form<S>() == 0) {
+                if constexpr (dev16_form<S, V>() == 0) {
                     float D0[Q], D1[Q];
 #pragma unroll
                     for (int i = 0; i < Q; ++i) {
@@ -705,7 +684,7 @@ __device__ __forceinline__ void update_vector(S (&fs)[Q][V], typename MapWord<V>
 #pragma unroll
                     for (int i = 0; i < Q; ++i)
                         D[i] = make_float2(Dev16<S>::to_f(fs[i][k]), Dev16<S>::to_f(fs[i][k + 1]));
-                    fluid_dev2<MODE != MODE_REDUCE, dev16_form<S>() == 2>(D, K, o0, o1);
+                    fluid_dev2<MODE != MODE_REDUCE>(D, K, o0, o1);
                     if (MODE != MODE_REDUCE) {
 #pragma unroll
                         for (int i = 0; i < Q; ++i) Dev16<S>::from_f2(D[i].x, D[i].y, fs[i][k], fs[i][k + 1]);

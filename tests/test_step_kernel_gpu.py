@@ -9,9 +9,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("prec", ["fp32", "fp64", "fp16", "bf16"])
-@pytest.mark.parametrize("dim,block", [(8, 0), (40, 0), (48, 32), (72, 0), (80, 256), (192, 0), (200, 0)])
+@pytest.mark.parametrize("dim,block", [(8, 0), (40, 0), (48, 32), (104, 0), (112, 256), (192, 0), (200, 0)])
 def test_step_shapes_agree(capi, prec, dim, block):
-    if prec == "fp64" and dim > 80:
+    if prec == "fp64" and dim > 104:
         pytest.skip("one shape for FP64")
     outs = []
     for kernel in ("auto", "aa"):
