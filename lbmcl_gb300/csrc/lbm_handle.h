@@ -98,6 +98,8 @@ struct lbm_handle {
     cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};
     cudaMemPool_t pool = nullptr;  // where its device memory comes from (null: cudaMalloc)
     bool pool_looked_up = false;
+    size_t pool_keep = 0;          // what that pool keeps when unused
+    std::vector<void *> plain;     // blocks from cudaMalloc beside it
     bool state_is_init = true;  // the populations are what lbm_init made
     size_t base_bytes = 0;      // device bytes lbm_init allocated
     lbm_adjoint_state adj;

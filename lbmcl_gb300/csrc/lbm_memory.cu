@@ -9,12 +9,18 @@
 //
 // The pool is the library's own, not the device's default one.  It keeps at
 // most a quarter of the device's memory once the handles are gone (its release
-// threshold; what is beyond goes back at the next synchronisation), and what it
+// threshold), and a block that would take it beyond that is a cudaMalloc of its
+// own: the pool maps new memory at 1.0 ms per GB and would unmap it at 0.7 on
+// every such use (cudaMalloc 0.03, cudaFree 0.33), and its blocks of 80 GB and
+// more are read slower.  256^3 backward sweeps, total ms from handle to handle,
+// FP16 T = 2000 with 250 GB: all from the pool 1912, with this rule 1539, all from
+// cudaMalloc 1645; FP32 T = 400 with 110 GB: 414, 355, 406.  What the pool
 // keeps is still there for the rest of the process: an allocation that does
 // not fit beside it makes the driver release it (measured: cudaMalloc of 266
 // GB succeeds on a 296 GB device whose pool holds 50 GB).  Allocations and
 // frees are ordered on the handle's stream; the driver orders a block's next
 // user behind them, whatever its stream or thread.
+#include <algorithm>
 #include <cstdint>
 #include <map>
 #include <mutex>
@@ -28,6 +34,7 @@ namespace {
 struct DevicePool {
     cudaMemPool_t pool = nullptr;
     unsigned long long context = 0;  // the context the pool was made in
+    size_t keep = 0;                 // bytes it keeps when unused
 };
 
 std::mutex g_mu;
@@ -52,12 +59,13 @@ unsigned long long context_id()
 }
 
 // The pool of the current device (null: none, plain cudaMalloc then).
-cudaMemPool_t device_pool(int device)
+cudaMemPool_t device_pool(int device, size_t *keep_bytes)
 {
     const unsigned long long ctx = context_id();
     if (ctx == 0) return nullptr;
     std::lock_guard<std::mutex> lock(g_mu);
     DevicePool &d = g_pools[device];
+    *keep_bytes = d.keep;
     if (d.pool && d.context == ctx) return d.pool;
     d.pool = nullptr;
     int has = 0;
@@ -85,6 +93,7 @@ cudaMemPool_t device_pool(int device)
     }
     d.pool = pool;
     d.context = ctx;
+    d.keep = *keep_bytes = (size_t)keep;
     return pool;
 }
 
@@ -95,17 +104,31 @@ namespace lbm {
 cudaError_t device_alloc(lbm_t *h, void **p, size_t bytes)
 {
     if (!h->pool_looked_up) {
-        h->pool = device_pool(h->cfg.device);
+        h->pool = device_pool(h->cfg.device, &h->pool_keep);
         h->pool_looked_up = true;
     }
-    return h->pool ? cudaMallocFromPoolAsync(p, bytes, h->pool, h->stream) : cudaMalloc(p, bytes);
+    if (!h->pool) return cudaMalloc(p, bytes);
+    uint64_t used = 0;
+    if (cudaMemPoolGetAttribute(h->pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
+        used + bytes > h->pool_keep) {
+        const cudaError_t e = cudaMalloc(p, bytes);
+        if (e == cudaSuccess) h->plain.push_back(*p);
+        if (e != cudaErrorMemoryAllocation) return e;
+        cudaGetLastError();  // perhaps beside blocks whose frees are still queued: the pool waits for those
+    }
+    return cudaMallocFromPoolAsync(p, bytes, h->pool, h->stream);
 }
 
 void device_free(lbm_t *h, void *p)
 {
     if (!p) return;
-    if (h->pool) cudaFreeAsync(p, h->stream);
-    else cudaFree(p);
+    const auto own = std::find(h->plain.begin(), h->plain.end(), p);
+    if (own != h->plain.end()) h->plain.erase(own);
+    else if (h->pool) {
+        cudaFreeAsync(p, h->stream);
+        return;
+    }
+    cudaFree(p);
 }
 
 size_t device_cached(const lbm_t *h)

@@ -78,3 +78,27 @@ def test_recorded_states_are_exact(capi, prec, steps, dim, iters, every):
                 np.testing.assert_array_equal(a[1], b[1])
                 np.testing.assert_array_equal(a[3], b[3])
                 np.testing.assert_array_equal(a[4], b[4])
+
+
+@pytest.mark.parametrize("first_out", [0, 1])
+def test_blocks_beyond_what_the_pool_keeps(capi, first_out):
+    """Two handles of 46 GB pass the quarter of the device's memory that the
+    pool keeps: a lattice of the second one has its own allocation, gives the
+    same state, and goes back when its handle does."""
+    torch = pytest.importorskip("torch")
+    free, total = torch.cuda.mem_get_info(0)
+    if total / 4 > 90e9 or free < 120e9:
+        pytest.skip("sized for a 280 GB device")
+    pair = [capi.Lattice(512, 0.005, 0.08, precision="fp64", seed=3, noise_sigma=1e-4) for _ in range(2)]
+    for L in pair:
+        L.step(2, every=2)
+    a, b = (L.reduce() for L in pair)
+    assert a == b
+    np.testing.assert_array_equal(pair[0].rho().view(np.uint64), pair[1].rho().view(np.uint64))
+    pair[first_out].close()
+    left = pair[1 - first_out]
+    left.step(1)
+    assert left.reduce() != a
+    left.close()
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info(0)[0] <= total / 4 + 2e9
