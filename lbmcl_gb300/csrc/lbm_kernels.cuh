@@ -1383,21 +1383,51 @@ template <class T> __device__ __forceinline__ void store4(T *p, const T (&v)[4])
     }
 }
 
-// Grid: blockIdx.y = z-plane, x-blocks over the plane's dim^2 / 4 groups of
-// four consecutive x-sites (dim % 4 == 0; 32-bit index arithmetic inside a
-// plane).  Each thread writes its four sites' map bytes, rho and u with one
-// vector store per field; the population slots of sites whose neighbours
-// are all FLUID take a branch-free path (nothing with noise, the rest state
-// without), the others init_site_pops.
+// Grid: blockIdx.y = z-plane, the six planes within three of a wall first.
+// The first nb x-blocks cover the plane's dim^2 / 4 groups of four consecutive
+// x-sites (dim % 4 == 0; 32-bit index arithmetic inside a plane): each thread
+// writes its four sites' map bytes, rho and u with one vector store per field,
+// and without noise the population slots of sites whose neighbours are all
+// FLUID.  The plane's other blocks write the population slots of its sites
+// within three of a wall (init_site_pops), a thread per site: the six row ends
+// and the rows near the y-faces, or all of a plane near a z-face.  In the
+// groups' threads nearly every warp held one row end and ran init_site_pops up
+// to three times for that one lane: the handle's creation took 1.08 ms at 256^3
+// FP16 with noise, now 0.88; in a kernel of their own the row ends' sectors
+// were written twice (without noise 0.50 ms, now 0.37, before 0.49).
 template <class S>
-__global__ void init_kernel(InitArgs a)
+__global__ void init_kernel(InitArgs a, unsigned nb)
 {
     using C = typename Compute<S>::type;
     const int dim = a.dim;
     const unsigned nq = (unsigned)dim / 4u;
+    const unsigned m = dim > 6 ? (unsigned)dim - 6u : 0u;  // y, z (and x) away from the walls: [3, dim-4]
+    const int z = m == 0 || blockIdx.y < 3 ? (int)blockIdx.y
+                : blockIdx.y < 6           ? (int)(blockIdx.y + m)
+                                           : (int)blockIdx.y - 3;
+    const bool inner = z >= 3 && z <= dim - 4;
+    if (blockIdx.x >= nb) {
+        const unsigned d = (unsigned)dim, ends = inner ? 6 * m : 0, count = inner ? ends + 6 * d : d * d;
+        for (unsigned t = (blockIdx.x - nb) * blockDim.x + threadIdx.x; t < count;
+             t += (gridDim.x - nb) * blockDim.x) {
+            unsigned x, y;
+            if (t < ends) {
+                const unsigned e = t % 6;
+                x = e < 3 ? e : m + e;
+                y = 3 + t / 6;
+            } else {
+                const unsigned r = (t - ends) / d;
+                x = t - ends - r * d;
+                y = inner && r >= 3 ? m + r : r;
+            }
+            init_site_pops<S>(a, (int)x, (int)y, z, ((size_t)z * d + y) * d + x,
+                              pack_cell(dim, (int)x, (int)y, z));
+        }
+        return;
+    }
     const unsigned pi = blockIdx.x * blockDim.x + threadIdx.x;
     if (pi >= nq * (unsigned)dim) return;
-    const int y = (int)(pi / nq), x0 = 4 * (int)(pi - (unsigned)y * nq), z = (int)blockIdx.y;
+    const int y = (int)(pi / nq), x0 = 4 * (int)(pi - (unsigned)y * nq);
     const size_t id0 = (size_t)z * dim * dim + (size_t)y * dim + (size_t)x0;
     uint8_t b[4];
 #pragma unroll
@@ -1420,48 +1450,28 @@ __global__ void init_kernel(InitArgs a)
     store4<C>(u + a.n + id0, u0);
     store4<C>(u + 2 * a.n + id0, u0);
 
-    // With noise, noise_kernel writes every slot whose value belongs to a
-    // FLUID site (the slots streaming into it, or its own in A-form); this
-    // kernel writes the others.
-    const bool noisy = a.noise_sigma != 0.0;
-    const bool bulk = y >= 3 && z >= 3 && y <= dim - 4 && z <= dim - 4;
-    if (bulk && x0 >= 3 && x0 + 3 <= dim - 4) {
-        // every site and all its neighbours are FLUID: the rest state
-        if (!noisy) {
-            S *f = static_cast<S *>(a.f);
-            const Weights<C> W = make_weights<C>();
+    // the rest state; with noise noise_kernel writes these slots
+    if (a.noise_sigma != 0.0 || !inner || y < 3 || y > dim - 4) return;
+    S *f = static_cast<S *>(a.f);
+    const Weights<C> W = make_weights<C>();
+    auto rest = [&](int i) -> S {
+        if constexpr (is_dev16<S>()) return Dev16<S>::from_f(0.0f);
+        else return (S)W.w[wclass_of(i)];
+    };
+    if (x0 >= 3 && x0 + 3 <= dim - 4) {
 #pragma unroll
-            for (int i = 0; i < Q; ++i) {
-                S v[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    if constexpr (is_dev16<S>()) v[k] = Dev16<S>::from_f(0.0f);
-                    else v[k] = (S)W.w[wclass_of(i)];
-                }
-                store4<S>(f + (size_t)i * a.n + id0, v);
-            }
+        for (int i = 0; i < Q; ++i) {
+            const S v[4] = {rest(i), rest(i), rest(i), rest(i)};
+            store4<S>(f + (size_t)i * a.n + id0, v);
         }
         return;
     }
 #pragma unroll 1
-    for (int k = 0; k < 4; ++k) {
-        const int x = x0 + k;
-        if (bulk && x >= 3 && x <= dim - 4) {
-            if (!noisy) {
-                S *f = static_cast<S *>(a.f);
-                const Weights<C> W = make_weights<C>();
+    for (int k = 0; k < 4; ++k)
+        if (x0 + k >= 3 && x0 + k <= dim - 4)
 #pragma unroll
-                for (int i = 0; i < Q; ++i) {
-                    if constexpr (is_dev16<S>()) f[(size_t)i * a.n + id0 + k] = Dev16<S>::from_f(0.0f);
-                    else f[(size_t)i * a.n + id0 + k] = (S)W.w[wclass_of(i)];
-                }
-            }
-            continue;
-        }
-        init_site_pops<S>(a, x, y, z, id0 + k, b[k]);
-    }
+            for (int i = 0; i < Q; ++i) f[(size_t)i * a.n + id0 + k] = rest(i);
 }
-
 
 // Seeded N(0, sigma^2) noise on the initial populations of the FLUID sites
 // (x, y, z in [2, dim-3]), run after init_kernel: the thread of FLUID site t

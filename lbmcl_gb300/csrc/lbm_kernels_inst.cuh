@@ -1,6 +1,8 @@
 // lbm_kernels_inst.cuh -- instantiates the kernels of one storage type.
 // Included by lbm_kernels_<type>.cu with LBM_S (element type), LBM_T (F-dump
 // element type) and LBM_SFX (launcher suffix) defined.
+#include <algorithm>
+
 #include "lbm_kernels.cuh"
 #include "lbm_launch.h"
 
@@ -173,9 +175,12 @@ const void *LBM_CAT(staged_kernel_ptr_, LBM_SFX)(int mode)
 cudaError_t LBM_CAT(launch_init_, LBM_SFX)(const InitArgs &a, cudaStream_t s)
 {
     const unsigned block = 256;
-    // four consecutive x-sites per thread (dim % 4 == 0)
-    const dim3 grid((unsigned)(((size_t)a.dim * a.dim / 4 + block - 1) / block), (unsigned)a.dim);
-    init_kernel<LBM_S><<<grid, block, 0, s>>>(a);
+    // four consecutive x-sites per thread (dim % 4 == 0), and the sites near the
+    // walls: 12 d of most planes, all d^2 of six (a thread each up to 90^3, then
+    // in turns: empty blocks elsewhere would cost more)
+    const unsigned d = (unsigned)a.dim, nb = (d * d / 4 + block - 1) / block;
+    const unsigned ns = std::min((d * d + block - 1) / block, std::max((12 * d + block - 1) / block, 32u));
+    init_kernel<LBM_S><<<dim3(nb + ns, d), block, 0, s>>>(a, nb);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || a.noise_sigma == 0.0 || a.dim < 5) return e;
     const size_t m = (size_t)(a.dim - 4);
