@@ -198,7 +198,10 @@ __device__ __forceinline__ A adjoint_fluid_core(A (&b)[Q], A ux, A uy, A uz, A o
 // A FLUID site's pre-collision populations g (adjoint type) and its moments
 // as the forward's collision formed them from the stored values v: the
 // deviation-form sums for 16-bit storage (moments_dev), the reference's
-// summation order for FP32 / FP64 (moments_exact).
+// summation order for FP32 / FP64 (moments_exact; the quotients from one
+// reciprocal: FP32 storage with a tau gradient, us per backward iteration with
+// three divisions -> this: 32^3 5.8 -> 4.8, 64^3 14.4 -> 12.4, 128^3 99.1 -> 83.7,
+// two steps per launch 256^3 909 -> 848; FP64 32^3 27.7 -> 24.5, 64^3 153.5 -> 133).
 template <class S, class A>
 __device__ __forceinline__ void forward_point(const S (&v)[Q], A (&g)[Q], A &rho, A &ux, A &uy, A &uz)
 {
@@ -220,7 +223,7 @@ __device__ __forceinline__ void forward_point(const S (&v)[Q], A (&g)[Q], A &rho
 #pragma unroll
         for (int i = 0; i < Q; ++i) f[i] = (C)v[i];
         C r, x, y, z;
-        moments_exact(f, r, x, y, z);
+        moments_exact<true>(f, r, x, y, z);
         rho = (A)r;
         ux = (A)x;
         uy = (A)y;
@@ -435,8 +438,20 @@ __device__ __forceinline__ void adjoint_vector(const AdjArgs &a, int xv, int y, 
 // 14.4 -> 7.1, 96^3 32 -> 22.6, 128^3 (FP16; from two steps per launch) 58.7
 // -> 51.4.  One site per thread instead of two: 64^3 7.2, 128^3 54.6, 256^3
 // 413 against 393.
+// Registers: 128 (with 16-bit states 168 are slower, 128^3 85 against 71 us),
+// FP64 no cap, FP32 states 168: both sites' 76 values stay in registers, 48^3
+// 6.4 against 7.7 us with 128, 64^3 12.3 / 12.4, 128^3 84.1 / 83.7.
+template <class S, class A, bool MACRO> __host__ __device__ constexpr int adj_threads()
+{
+    return sizeof(A) == 4 && sizeof(S) == 4 && !MACRO ? 128 : 256;
+}
+template <class S, class A, bool MACRO> __host__ __device__ constexpr int adj_min_blocks()
+{
+    return sizeof(A) == 8 ? 1 : sizeof(S) == 4 && !MACRO ? 3 : 2;
+}
 template <class S, class A, bool MACRO>
-__global__ void __launch_bounds__(256, sizeof(A) == 8 ? 1 : 2) adjoint_kernel(AdjArgs a, StepRows r)
+__global__ void __launch_bounds__(adj_threads<S, A, MACRO>(), adj_min_blocks<S, A, MACRO>())
+    adjoint_kernel(AdjArgs a, StepRows r)
 {
     constexpr int V = ADJ_VB / (int)sizeof(A);
     const int dim = a.dim;

@@ -243,9 +243,21 @@ __device__ __forceinline__ void moments_sailfish(const T (&f)[Q], T &r, T &ux, T
     uz = O::div(s, r);
 }
 
+// n / d from y = 1 / d rounded to nearest: Markstein's correction (IBM Journal
+// of Research and Development 34, 1990) gives the rounded quotient, in the
+// normal range and but for a last bit where d's mantissa is all ones.
+__device__ __forceinline__ float rcp_rn(float d) { return __frcp_rn(d); }
+__device__ __forceinline__ double rcp_rn(double d) { return __drcp_rn(d); }
+template <class T> __device__ __forceinline__ T quot_rcp(T n, T d, T y)
+{
+    const T q = X<T>::mul(n, y);
+    return fma(fma(-q, d, n), y, q);
+}
+
 // Density (kernels.cl:355) and momentum sums (kernels.cl:376-378) in the
-// reference's summation order.
-template <class T>
+// reference's summation order.  ONE_RCP: the three quotients from one
+// reciprocal, without the branches of three divisions.
+template <bool ONE_RCP = false, class T>
 __device__ __forceinline__ void moments_exact(const T (&f)[Q], T &r, T &ux, T &uy, T &uz)
 {
     using O = X<T>;
@@ -258,9 +270,16 @@ __device__ __forceinline__ void moments_exact(const T (&f)[Q], T &r, T &ux, T &u
     const T my = O::add(O::add(O::add(O::add(f[4], f[9]), f[10]), f[14]), f[18]);
     const T pz = O::add(O::add(O::add(O::add(f[6], f[15]), f[16]), f[17]), f[18]);
     const T mz = O::add(O::add(O::add(O::add(f[5], f[11]), f[12]), f[13]), f[14]);
-    ux = O::div(O::sub(px, mx), r);
-    uy = O::div(O::sub(py, my), r);
-    uz = O::div(O::sub(pz, mz), r);
+    if constexpr (ONE_RCP) {
+        const T y = rcp_rn(r);
+        ux = quot_rcp(O::sub(px, mx), r, y);
+        uy = quot_rcp(O::sub(py, my), r, y);
+        uz = quot_rcp(O::sub(pz, mz), r, y);
+    } else {
+        ux = O::div(O::sub(px, mx), r);
+        uy = O::div(O::sub(py, my), r);
+        uz = O::div(O::sub(pz, mz), r);
+    }
 }
 
 // Equilibrium of a site at rest density 1 moving with (lid, 0, 0): the value
