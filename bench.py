@@ -277,7 +277,8 @@ def time_adjoint(capi, prec, device, with_tau=False):
         L.step(T)
         L.step(1, every=T + 1)
         target = np.nan_to_num(L.u().reshape(3, dim, dim, dim)[0, :, a["plane_y"], :]).reshape(-1)
-    free0 = torch.cuda.mem_get_info(device)[0]
+    # (of all the device's memory: the handles' pool keeps idle blocks between legs)
+    total = torch.cuda.mem_get_info(device)[1]
     with capi.Lattice(dim, a["viscosity"], 0.0, precision=prec, lid=lid, stride=0, device=device) as L:
         stream = torch.cuda.ExternalStream(L.stream, device=device)
         L.step(5)
@@ -316,7 +317,7 @@ def time_adjoint(capi, prec, device, with_tau=False):
             "checkpointed_forward_ms_per_iter": round(ckpt_ms, 4), "backward_ms_per_iter": round(bwd_ms, 4),
             "adjoint_over_forward": round(bwd_ms / fwd_ms, 3),
             "forward_plus_backward_over_forward": round((ckpt_ms + bwd_ms) / fwd_ms, 3),
-            "device_gb_peak": round((free0 - min(free1, free2)) / 1e9, 1)}
+            "device_gb_peak": round((total - min(free1, free2)) / 1e9, 1)}
 
 
 def traffic_from_profiles(prec):
@@ -546,7 +547,8 @@ def main():
                     "d2h_bytes_per_step": d2h / args.steps,
                     "what": "lbm_init (host config + lid profile) + K iterations + rho/u read-back to pinned host",
                     "parts": e2e_parts},
-            "gpu_launches": 2 * args.steps * res[head]["windows"],
+            # 16-bit storage at this size: two launches an iteration, FP32 / FP64 one
+            "gpu_launches": (2 if head in ("fp16", "bf16") else 1) * args.steps * res[head]["windows"],
             "timed_windows": {"windows": res[head]["windows"], "steps_per_window": args.steps,
                               "reported": "median window"},
             "clocks": sampler.summary(),

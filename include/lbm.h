@@ -98,11 +98,11 @@ typedef struct lbm_config {
     int profile_steps;         /* 1: one CUDA event pair per iteration (reference's
                                   per-kernel events); 0: one pair per lbm_step call         */
     int kernel;                /* lbm_kernel: iteration kernel variant; 0 = the tuned default
-                                  (NARROW for FP32, DIRECT otherwise)                       */
+                                  (vector width by storage type and lattice size)           */
     int stages;                /* TMA-staged kernel: pipeline depth (0 = tuned default)    */
     int adjoint_steps;         /* adjoint steps per launch of the backward sweep: 0 = tuned
-                                  default (2 for the FP32 adjoint on lattices that fill the
-                                  GPU, about 128^3 and up; else 1), 1, or 2 (FP32 adjoint,
+                                  default (2 for the FP32 adjoint beyond 192^3; else 1), 1,
+                                  or 2 (FP32 adjoint,
                                   dim <= 609)                                               */
     int adjoint_max_states;    /* > 0: at most this many recomputed state buffers in the
                                   backward sweep (fewer than checkpoint_every - 1 makes it

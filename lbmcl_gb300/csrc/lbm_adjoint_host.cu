@@ -8,8 +8,8 @@
 // a_T = dJ/dR_T, then walks the segments backwards: it restores a
 // checkpoint, recomputes the segment's intermediate states with the forward
 // kernel, and applies the adjoint step from the segment's last iteration to
-// its first, two steps per launch for the FP32 adjoint (a segment of odd
-// length ends with one single step).  When the segment's states do not fit
+// its first, two steps per launch for the FP32 adjoint beyond 192^3 (a segment
+// of odd length ends with one single step).  When the segment's states do not fit
 // in device memory, the segment itself is checkpointed and swept recursively
 // (one more forward pass per level).  Memory: ceil(T/c) checkpoints + (c - 1) segment states, i.e.
 // about 2 sqrt(T) states for c = sqrt(T); one extra forward iteration per
