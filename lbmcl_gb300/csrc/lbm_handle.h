@@ -75,6 +75,9 @@ struct lbm_handle {
     // rows) and its fork / join events
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    // copies of F dumps and loads beside their kernels, made by the first one
+    cudaStream_t copy = nullptr;
+    std::vector<cudaEvent_t> copy_events;
     cudaEvent_t ev_first = nullptr, ev_last = nullptr;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> pending;
     std::vector<cudaEvent_t> spare;
