@@ -5,9 +5,9 @@
 // Bound: the FP64 pipe.  GB300 runs an FP64 operation for one warp in 16 to 20
 // cycles per SM, and 64 to 128 lanes of integer adds, logic or products a
 // cycle beside it; the update is 260 FP64 operations a site in IEEE operations,
-// 80 here, and 4,500 integer instructions.  256^3: 7767 -> 3777 us per
-// iteration (2110 -> 4339 MLUPS, 9% -> 19% of HBM), 64^3 133 -> 66, 16^3 13.3 ->
-// 10.4 (ncu at 128^3: FP64 pipe 64% active, integer pipe 60%).  The last sum of
+// 80 here, and 4,500 integer instructions.  256^3: 7767 -> 3470 us per
+// iteration (2110 -> 4722 MLUPS, 9% -> 21% of HBM), 64^3 133 -> 62.9, 32^3 19.6 ->
+// 12.0 (ncu at 128^3: FP64 pipe 64% active, integer pipe 60%).  The last sum of
 // every population on the FP64 pipe too (19 operations more, a seventh of the
 // integer instructions less): 256^3 4436.  At 128 registers, 16 warps per SM
 // (254 registers, 8 warps: 4698; 80 registers with spills: 3779).
@@ -24,11 +24,15 @@
 // jammed into the lowest one ("round to odd"): where they do, at least two bits
 // are dropped, so the lowest one only has to say "not exact".
 //
-// The windows (f_0 in [2^-8, 1), f_i in [2^-8, 1/4), new f_i at least 2^-7,
-// |u_x|, |u_y|, |u_z| < 1/8, rho in [7/8, 2), feq - f a double, as it is within a
-// factor of two, |feq - f| / tau < 1/2, 2^-10 <= 1/tau < 64) hold for
-// flows well inside the low-Mach range of the scheme; a site outside any of
-// them reports false and takes the IEEE path.
+// The windows (f_0 in [2^-8, 1), f_i in [2^-8, 1/4), 2^-10 <= 1/tau < 64; then
+// rho in [7/8, 2), |u_x|, |u_y|, |u_z| < 1/8; then feq - f a double, as it is within
+// a factor of two, |feq - f| / tau < 1/2, new f in [2^-7, 2)) hold for flows well
+// inside the low-Mach range of the scheme.  Beyond the first the update is IEEE
+// operations (260), beyond the others its relaxation is (170 beside the 18 of
+// the moments here), so that a site outside takes no longer than without all
+// this: 256^3 with |u| = 0.15 everywhere 5933 us per iteration, rho = 2.5 5935,
+// IEEE operations alone 8431 (both updates one after the other 9663, 9089).  The
+// lanes of a warp leave together: some inside and some outside would run both.
 #pragma once
 
 #include "lbm_device.cuh"
@@ -161,9 +165,16 @@ __device__ __forceinline__ double relaxed(double feq, u64 F, double inv_tau, Ext
     return to_double(S);
 }
 
-// The BGK update of a FLUID site (f in and out) and its moments.  False: some
-// window did not hold, f is not valid then.
-__device__ __forceinline__ bool fluid(double (&f)[Q], double inv_tau, const Weights<double> &W, double &r_, double &ux_,
+// What fluid did: nothing (f as it was), the moments (f not valid), or the
+// moments and the update.
+enum Done { NOTHING, MOMENTS, UPDATE };
+
+// Does any lane of the warp (of those here) say so?
+__device__ __forceinline__ bool any(bool p) { return __any_sync(__activemask(), p); }
+
+// The BGK update of a FLUID site (f in and out) and its moments, as far as the
+// windows let it.
+__device__ __forceinline__ Done fluid(double (&f)[Q], double inv_tau, const Weights<double> &W, double &r_, double &ux_,
                                       double &uy_, double &uz_)
 {
     unsigned least = hi32(bits(f[1])), most = least;
@@ -173,9 +184,9 @@ __device__ __forceinline__ bool fluid(double (&f)[Q], double inv_tau, const Weig
         most = max(most, hi32(bits(f[i])));
     }
     // (a set sign makes a high word larger than any of these bounds)
-    if (least < (1015u << 20) || most >= (1021u << 20) || hi32(bits(f[0])) - (1015u << 20) >= (8u << 20) ||
-        hi32(bits(inv_tau)) - (1013u << 20) >= (16u << 20))
-        return false;
+    if (any(least < (1015u << 20) || most >= (1021u << 20) || hi32(bits(f[0])) - (1015u << 20) >= (8u << 20) ||
+            hi32(bits(inv_tau)) - (1013u << 20) >= (16u << 20)))
+        return NOTHING;
     u64 F[Q];
 #pragma unroll
     for (int i = 0; i < Q; ++i) F[i] = exact(f[i]);
@@ -191,14 +202,18 @@ __device__ __forceinline__ bool fluid(double (&f)[Q], double inv_tau, const Weig
     const double pz = to_double(round53(round53(round53(F[6] + F[15]) + F[16]) + F[17]) + F[18]);
     const double mz = to_double(round53(round53(round53(F[5] + F[11]) + F[12]) + F[13]) + F[14]);
     double ux, uy, uz;
+    // (r is at least 19 2^-8 and below 5.5; a difference is a multiple of 2^-61)
     quotients(__dsub_rn(px, mx), __dsub_rn(py, my), __dsub_rn(pz, mz), r, ux, uy, uz);
+    r_ = r;
+    ux_ = ux;
+    uy_ = uy;
+    uz_ = uz;
     const unsigned top = 1020u << 20;  // 1/8
     // rho in [7/8, 2): with |u_i| < 1/8 every bracket is at least 0.46 and
     // every feq at least 0.011
-    if ((hi32(bits(ux)) & 0x7fffffffu) >= top || (hi32(bits(uy)) & 0x7fffffffu) >= top ||
-        (hi32(bits(uz)) & 0x7fffffffu) >= top || hi32(bits(r)) - 0x3fec0000u >= 0x40000000u - 0x3fec0000u)
-        return false;
-    bool ok = true;
+    if (any((hi32(bits(ux)) & 0x7fffffffu) >= top || (hi32(bits(uy)) & 0x7fffffffu) >= top ||
+            (hi32(bits(uz)) & 0x7fffffffu) >= top || hi32(bits(r)) - 0x3fec0000u >= 0x40000000u - 0x3fec0000u))
+        return MOMENTS;
     Extremes x;
     const double u2 = __dadd_rn(__dadd_rn(__dmul_rn(ux, ux), __dmul_rn(uy, uy)), __dmul_rn(uz, uz));
     const u64 C = jam(__dmul_rn(1.5, u2));
@@ -212,7 +227,7 @@ __device__ __forceinline__ bool fluid(double (&f)[Q], double inv_tau, const Weig
         const u64 b = bits(eu);
         const unsigned sign = hi32(b) & 0x80000000u, e = (hi32(b) >> 20) & 0x7ffu;
         const u64 m = make64((hi32(b) & 0xfffffu) | 0x100000u, lo32(b));
-        ok &= e != 0 || (b << 1) == 0;
+        // (a subnormal eu gives what zero gives)
         // |3 eu|: 3 m has 54 or 55 bits
         const u64 m3 = 3 * m;
         const int t3 = 1 + (int)(hi32(m3) >> 22);
@@ -228,14 +243,13 @@ __device__ __forceinline__ bool fluid(double (&f)[Q], double inv_tau, const Weig
         const double w = rw[wclass_of(i)];
         f[i] = relaxed(__dmul_rn(w, sign ? minus : plus), F[i], inv_tau, x);
         f[j] = relaxed(__dmul_rn(w, sign ? plus : minus), F[j], inv_tau, x);
+        // (most sites that fail below fail here)
+        if (any((x.lost & 0x7ffu) != 0)) return MOMENTS;
     }
-    r_ = r;
-    ux_ = ux;
-    uy_ = uy;
-    uz_ = uz;
     // every feq - f a double, every change below 1/2, 2^-7 <= new f (two bits
     // dropped) < 2
-    return ok && (x.lost & 0x7ffu) == 0 && x.change < (1022u << 20) && x.least >= (1u << 22) && x.most < (1u << 30);
+    const bool ok = x.change < (1022u << 20) && x.least >= (1u << 22) && x.most < (1u << 30);
+    return any(!ok) ? MOMENTS : UPDATE;
 }
 
 }  // namespace fx

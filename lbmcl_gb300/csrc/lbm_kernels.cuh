@@ -709,24 +709,35 @@ __device__ __forceinline__ void update_vector(S (&fs)[Q][V], typename MapWord<V>
 }
 
 
-// update_vector of one FP64 site of an interior row in 64-bit integers where
-// they serve (fx::fluid): the same bits.  False: not done, fs not valid.  The
+// update_vector of one FP64 site of an interior row, in 64-bit integers as far
+// as they serve (fx::fluid) and in IEEE operations beyond: the same bits.  The
 // row ends are not FLUID: nothing to do (face_fix, and walls nobody reads).
 template <int MODE>
-__device__ __forceinline__ bool update_fixed(double (&fs)[Q][1], const StepArgs &a, int x0, size_t site0)
+__device__ __forceinline__ void update_fixed(double (&fs)[Q][1], const StepArgs &a, size_t rowoff, int x0, size_t site0)
 {
-    if ((unsigned)(x0 - 2) > (unsigned)(a.dim - 5)) return true;
-    if (a.sailfish) return false;
+    if ((unsigned)(x0 - 2) > (unsigned)(a.dim - 5)) return;
     double f[Q];
 #pragma unroll
     for (int i = 0; i < Q; ++i) f[i] = fs[i][0];
+    const Weights<double> W = make_weights<double>();
     SiteOut o;
-    if (!fx::fluid(f, a.inv_tau, make_weights<double>(), o.r, o.ux, o.uy, o.uz)) return false;
+    const fx::Done d = a.sailfish ? fx::NOTHING : fx::fluid(f, a.inv_tau, W, o.r, o.ux, o.uy, o.uz);
+    if (d != fx::UPDATE) {
+        if (d == fx::MOMENTS) {
+            gather_all<double, 1, 0, false>(static_cast<const double *>(a.fin), a.n, rowoff, a.dim, x0, fs);
+#pragma unroll
+            for (int i = 0; i < Q; ++i) f[i] = fs[i][0];
+        } else {
+            if (a.sailfish) moments_sailfish(f, o.r, o.ux, o.uy, o.uz);
+            else moments_exact(f, o.r, o.ux, o.uy, o.uz);
+            if (!(o.r > 0.0)) atomicOr(a.status, 1);
+        }
+        relax_exact(f, o.r, o.ux, o.uy, o.uz, a.inv_tau, W);
+    }
 #pragma unroll
     for (int i = 0; i < Q; ++i) fs[i][0] = f[i];
     if (MODE == MODE_STEP_MACRO) store_macro<double>(a, site0, o);
     if (MODE == MODE_STEP_ADJ) store_adj<double>(a, site0, o, false);
-    return true;
 }
 
 // Bounce-back of the x-face site x = xf of an interior row (y, z in
@@ -770,12 +781,10 @@ __device__ __forceinline__ void pull_vector(const StepArgs &a, int xv, int y, in
     const S *__restrict__ fin = static_cast<const S *>(a.fin);
     S fs[Q][V];
     gather_all<S, V, 0, NC>(fin, a.n, rowoff, dim, x0, fs);
-    bool done = false;
-    if constexpr (std::is_same<S, double>::value && V == 1 && INTERIOR && MODE != MODE_REDUCE) {
-        done = update_fixed<MODE>(fs, a, x0, site0);
-        if (!done) gather_all<S, V, 0, NC>(fin, a.n, rowoff, dim, x0, fs);
-    }
-    if (!done) update_vector<S, MODE, V, INTERIOR>(fs, mw, a, y, z, x0, site0, red_m, red_e);
+    if constexpr (std::is_same<S, double>::value && V == 1 && INTERIOR && MODE != MODE_REDUCE)
+        update_fixed<MODE>(fs, a, rowoff, x0, site0);
+    else
+        update_vector<S, MODE, V, INTERIOR>(fs, mw, a, y, z, x0, site0, red_m, red_e);
     if (INTERIOR && MODE != MODE_REDUCE) {
         // the walls (x = 0, dim-1) hold values nobody reads; the faces bounce back
         if constexpr (V == 1) {
