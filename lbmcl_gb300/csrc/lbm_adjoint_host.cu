@@ -901,6 +901,7 @@ int lbm_adjoint_backward(lbm_t *h, double dloss, double *grad_tau, double *grad_
     if (grad_f0) {
         const size_t total = (size_t)lbm::Q * h->n;
         const size_t chunk = std::min(total, (size_t)1 << 25);
+        const bool pages = total > chunk && !lbm::page_locked(grad_f0, total * db);
         for (size_t o0 = 0; o0 < total; o0 += chunk) {
             const size_t cnt = std::min(chunk, total - o0);
             const unsigned g = (unsigned)((cnt + 255) / 256);
@@ -914,6 +915,7 @@ int lbm_adjoint_backward(lbm_t *h, double dloss, double *grad_tau, double *grad_
                 lbm::export_adjoint_kernel<float, float><<<g, 256, 0, st>>>(
                     static_cast<const float *>(s.adj[cur]), static_cast<float *>(h->stage), o0, cnt, h->sd, h->n);
             ADJ_CUDA(cudaGetLastError());
+            if (pages) lbm::make_pages((char *)grad_f0 + o0 * db, cnt * db);
             ADJ_CUDA(cudaMemcpyAsync((char *)grad_f0 + o0 * db, h->stage, cnt * db, cudaMemcpyDeviceToHost, st));
         }
     }

@@ -20,6 +20,9 @@
 // GB succeeds on a 296 GB device whose pool holds 50 GB).  Allocations and
 // frees are ordered on the handle's stream; the driver orders a block's next
 // user behind them, whatever its stream or thread.
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <cstdint>
 #include <map>
@@ -100,6 +103,29 @@ cudaMemPool_t device_pool(int device, size_t *keep_bytes)
 }  // namespace
 
 namespace lbm {
+
+bool page_locked(const void *p, size_t bytes)
+{
+    for (const char *at : {static_cast<const char *>(p), static_cast<const char *>(p) + bytes - 1}) {
+        cudaPointerAttributes pa;
+        if (cudaPointerGetAttributes(&pa, at) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (pa.type != cudaMemoryTypeHost) return false;
+    }
+    return true;
+}
+
+void make_pages(void *host, size_t bytes)
+{
+#ifdef MADV_POPULATE_WRITE
+    // only a hint: the copies meet whatever pages it leaves
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), p = (uintptr_t)host;
+    const uintptr_t first = (p + page - 1) / page * page, last = (p + bytes) / page * page;
+    if (last > first) madvise((void *)first, last - first, MADV_POPULATE_WRITE);
+#endif
+}
 
 cudaError_t device_alloc(lbm_t *h, void **p, size_t bytes)
 {
