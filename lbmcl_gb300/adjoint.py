@@ -30,12 +30,15 @@ class _CavityLoss(torch.autograd.Function):
     def forward(ctx, lid, tau, f0, opts):
         dim = opts["dim"]
         # the forward records what the backward sweep needs of the last segments'
-        # iterations: their linearisation points, with a tau gradient their states
+        # iterations: their linearisation points, with a tau gradient their states,
+        # nothing where no sweep can follow
+        record = opts.get("grad_mode", True) and any(ctx.needs_input_grad)
         L = capi.Lattice(dim, velocity=0.0, precision=opts.get("precision", "fp32"),
                          stride=opts.get("stride"), lid=lid.detach().cpu().numpy().reshape(-1),
                          tau=float(tau), seed=opts.get("seed", 0), noise_sigma=opts.get("noise", 0.0),
                          device=opts.get("device", 0),
-                         adjoint_full_states=bool(ctx.needs_input_grad[1]))
+                         adjoint_full_states=bool(record and ctx.needs_input_grad[1]),
+                         adjoint_tail_segments=0 if record else -1)
         if f0 is not None:
             L.load_f(f0.detach().cpu().numpy())
         L.adjoint_set_loss(opts["plane_y"], opts.get("target"))
@@ -65,6 +68,8 @@ def cavity_loss(lid: torch.Tensor, tau: torch.Tensor, f0, *, dim: int, iteration
                 noise: float = 0.0, device: int = 0) -> torch.Tensor:
     """Mid-plane velocity loss of a `dim`^3 cavity after `iterations` steps
     (differentiable in lid, tau and f0)."""
+    # (inside forward the gradient mode is always off, and needs_input_grad does not depend on it)
     opts = dict(dim=dim, iterations=iterations, plane_y=plane_y, target=target, checkpoint_every=checkpoint_every,
-                precision=precision, stride=stride, seed=seed, noise=noise, device=device)
+                precision=precision, stride=stride, seed=seed, noise=noise, device=device,
+                grad_mode=torch.is_grad_enabled())
     return _CavityLoss.apply(lid, tau, f0, opts)
