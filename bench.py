@@ -269,6 +269,8 @@ def time_adjoint(capi, prec, device, with_tau=False):
     import torch
     from lbmcl_gb300.validate import smooth_lid
     a = ADJOINT_TAU if with_tau else (ADJOINT if prec in ("fp16", "bf16") else ADJOINT_FP32)
+    capi.keep_memory(0, device)  # what earlier legs left idle is not this one's
+    capi.keep_memory(None, device)
     dim, T, c = a["dim"], a["iterations"], a["checkpoint_every"]
     rng = np.random.default_rng(1234)
     target_lid = smooth_lid(dim, rng).reshape(-1)
@@ -277,7 +279,6 @@ def time_adjoint(capi, prec, device, with_tau=False):
         L.step(T)
         L.step(1, every=T + 1)
         target = np.nan_to_num(L.u().reshape(3, dim, dim, dim)[0, :, a["plane_y"], :]).reshape(-1)
-    # (of all the device's memory: the handles' pool keeps idle blocks between legs)
     total = torch.cuda.mem_get_info(device)[1]
     with capi.Lattice(dim, a["viscosity"], 0.0, precision=prec, lid=lid, stride=0, device=device) as L:
         stream = torch.cuda.ExternalStream(L.stream, device=device)

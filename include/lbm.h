@@ -93,7 +93,8 @@ typedef struct lbm_config {
                                   at lid_profile[x + y*dim]; NULL = velocity everywhere    */
     double tau;                /* > 0 overrides the viscosity                               */
     size_t max_device_bytes;   /* > 0: refuse (LBM_ENOMEM) when the handle would need
-                                  more device memory than this                              */
+                                  more device memory than this (what the library keeps
+                                  idle: lbm_keep_memory)                                    */
     int device;                /* CUDA device ordinal                                       */
     int profile_steps;         /* 1: one CUDA event pair per iteration (reference's
                                   per-kernel events); 0: one pair per lbm_step call         */
@@ -138,9 +139,10 @@ typedef struct lbm_config {
                                   0 = as many segments as fit in the device memory left
                                   beyond what the sweep itself needs, n > 0 = at most n,
                                   -1 = none; with adjoint_full_states it records the states
-                                  themselves (within a quarter of the device's memory), for
-                                  sweeps with or without a tau gradient; the gradients are
-                                  the same bit for bit                                     */
+                                  themselves (within a quarter of the device's memory for
+                                  all handles of the process together), for sweeps with or
+                                  without a tau gradient; the gradients are the same bit for
+                                  bit                                                       */
 } lbm_config;
 
 /* Iteration kernel variants (same results, different data movement). */
@@ -253,7 +255,20 @@ int lbm_adjoint_forward(lbm_t *h, int iterations, int checkpoint_every, double *
 int lbm_adjoint_backward(lbm_t *h, double dloss, double *grad_tau, double *grad_lid, void *grad_f0,
                          size_t grad_f0_bytes);
 
+/* Release the handle.  Its device memory stays with the library for the next
+ * handle on that device, up to lbm_keep_memory's limit for all handles of the
+ * process together; what is beyond goes back to the device now. */
 void lbm_destroy(lbm_t *h);
+
+/* Device memory that the library keeps on a device when its handles do not use
+ * it: at most `bytes` from now on ((size_t)-1, as at the start: a quarter of the
+ * device's memory).  What is idle beyond that goes back to the device before
+ * the call returns; with 0 everything a handle had goes back when it is
+ * destroyed.  Idle memory counts as used in cudaMemGetInfo and towards no
+ * handle's max_device_bytes; allocations of this process that would not fit
+ * beside it get it, other processes on the GPU do not.  May be called at any
+ * time, from any thread; handles in use are not affected. */
+int lbm_keep_memory(int device, size_t bytes);
 
 const char *lbm_last_error(void);
 

@@ -95,6 +95,7 @@ def lib():
     L.lbm_reduce.argtypes = [vp, C.POINTER(C.c_double)]
     L.lbm_destroy.argtypes = [vp]
     L.lbm_destroy.restype = None
+    L.lbm_keep_memory.argtypes = [C.c_int, sz]
     L.lbm_last_error.restype = C.c_char_p
     L.lbm_device_name.argtypes = [vp]
     L.lbm_device_name.restype = C.c_char_p
@@ -102,7 +103,7 @@ def lib():
     L.lbm_adjoint_forward.argtypes = [vp, C.c_int, C.c_int, C.POINTER(C.c_double)]
     L.lbm_adjoint_backward.argtypes = [vp, C.c_double, C.POINTER(C.c_double), C.POINTER(C.c_double), vp, sz]
     for name in ("lbm_init", "lbm_step", "lbm_dump", "lbm_load", "lbm_sync", "lbm_timing", "lbm_iteration",
-                 "lbm_reduce", "lbm_adjoint_set_loss", "lbm_adjoint_forward", "lbm_adjoint_backward"):
+                 "lbm_reduce", "lbm_keep_memory", "lbm_adjoint_set_loss", "lbm_adjoint_forward", "lbm_adjoint_backward"):
         getattr(L, name).restype = C.c_int
     _lib = L
     return L
@@ -117,6 +118,14 @@ def default_config() -> Config:
     c = Config()
     lib().lbm_config_default(C.byref(c))
     return c
+
+
+def keep_memory(nbytes=None, device: int = 0) -> None:
+    """Bytes of device memory the library keeps for the next handle when none
+    uses it (None: the default, a quarter of the device's memory; 0: a handle's
+    memory goes back to the device when it is closed).  What is idle beyond
+    that goes back now."""
+    check(lib().lbm_keep_memory(int(device), C.c_size_t(-1 if nbytes is None else int(nbytes))))
 
 
 class Lattice:

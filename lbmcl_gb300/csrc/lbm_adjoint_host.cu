@@ -626,10 +626,12 @@ int lbm_adjoint_forward(lbm_t *h, int iterations, int checkpoint_every, double *
     // to a buffer of its own).  As many as fit in the device memory left once
     // the sweep's own buffers (the checkpoints above, a segment's point sets or
     // states, two state scratch buffers, the staged checkpoint, the two adjoint
-    // buffers) are set aside.  States: within the quarter of the device's memory
-    // that the pool keeps from one handle to the next; mapping and unmapping one
-    // beyond it takes longer than the iteration it saves (256^3 FP16: 0.64 GB,
-    // 0.5 ms, against 0.21 ms).
+    // buffers) are set aside.  States: within a quarter of the device's memory
+    // for all of the process's handles together, so that several losses held at
+    // once still find room for their checkpoints, and as much as the pool keeps from
+    // one handle to the next unless told otherwise; mapping and unmapping one beyond
+    // it takes longer than the iteration it saves (256^3 FP16: 0.64 GB, 0.5 ms,
+    // against 0.21 ms).
     const bool states = h->cfg.adjoint_full_states != 0;
     const size_t mbytes = states ? fbytes : 3 * h->n * lbm::macro_bytes(h->prec);
     int mt = 0;
@@ -646,7 +648,7 @@ int lbm_adjoint_forward(lbm_t *h, int iterations, int checkpoint_every, double *
         if (states) {
             size_t freeb = 0, totalb = 0;
             if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) totalb = 0;
-            const size_t used = h->base_bytes + s.bytes;
+            const size_t used = lbm::device_in_use(h);
             r = std::min(r, totalb / 4 > used ? totalb / 4 - used : (size_t)0);
         }
         // with every segment recorded nothing of a segment's recompute is held

@@ -928,4 +928,14 @@ int lbm_reduce(lbm_t *h, double out[3])
 
 void lbm_destroy(lbm_t *h) { release(h); }
 
+int lbm_keep_memory(int device, size_t bytes)
+{
+    int count = 0;
+    LBM_CUDA(cudaGetDeviceCount(&count));
+    if (device < 0 || device >= count)
+        return fail(LBM_EINVAL, "lbm_keep_memory: device %d of %d", device, count);
+    LBM_CUDA(lbm::keep_memory(device, bytes));
+    return LBM_OK;
+}
+
 }  // extern "C"

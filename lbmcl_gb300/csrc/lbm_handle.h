@@ -101,8 +101,7 @@ struct lbm_handle {
     cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};
     cudaMemPool_t pool = nullptr;  // where its device memory comes from (null: cudaMalloc)
     bool pool_looked_up = false;
-    size_t pool_keep = 0;          // what that pool keeps when unused
-    std::vector<void *> plain;     // blocks from cudaMalloc beside it
+    std::vector<std::pair<void *, size_t>> plain;  // blocks from cudaMalloc beside it, their bytes
     bool state_is_init = true;  // the populations are what lbm_init made
     size_t base_bytes = 0;      // device bytes lbm_init allocated
     lbm_adjoint_state adj;
@@ -139,10 +138,13 @@ cudaError_t launch_iteration_adj(const lbm_t *h, const void *fin, void *fout, vo
 // (an even count: h->cur is unchanged)
 cudaError_t replay_iterations(lbm_t *h);
 // device memory of a handle, ordered on its stream (lbm_memory.cu); device_cached:
-// bytes its pool holds beside what is in use
+// bytes its pool holds beside what is in use; device_in_use: bytes that the
+// process's handles on its device have; keep_memory: lbm_keep_memory
 cudaError_t device_alloc(lbm_t *h, void **p, size_t bytes);
 void device_free(lbm_t *h, void *p);
 size_t device_cached(const lbm_t *h);
+size_t device_in_use(const lbm_t *h);
+cudaError_t keep_memory(int device, size_t bytes);
 // is [p, p + bytes) page-locked host memory?
 bool page_locked(const void *p, size_t bytes);
 // Make the pages of [host, host + bytes) that the process has not touched yet, for

@@ -225,6 +225,8 @@ def lidfield(args):
         fwd_ms = e0.elapsed_time(e1) / 100
 
     def run_adjoint(prec, every, a64=False):
+        capi.keep_memory(0)  # what earlier handles left idle is not this run's
+        capi.keep_memory()
         free0, _ = torch.cuda.mem_get_info()
         with capi.Lattice(dim, velocity=0.0, precision=prec, lid=lid, tau=tau, stride=0, adjoint_fp64=a64) as L:
             L.adjoint_set_loss(plane, target)
