@@ -296,8 +296,8 @@ int step_shape(int kernel, int prec, int dim)
 {
     const bool s16 = prec == LBM_FP16 || prec == LBM_BF16;
     if (kernel == LBM_KERNEL_NARROW) return 8;
-    if (kernel == LBM_KERNEL_DIRECT && !s16) return 16;
-    if (prec == LBM_FP64) return 8;
+    if (prec == LBM_FP64) return kernel == LBM_KERNEL_DIRECT ? 16 : 8;
+    if (kernel == LBM_KERNEL_DIRECT && !s16) return 0;
     if (prec == LBM_FP32) return dim <= 40 ? 4 : 8;
     if (dim > 192) return 0;
     if (kernel == LBM_KERNEL_DIRECT) return 16;
@@ -307,8 +307,11 @@ int step_shape(int kernel, int prec, int dim)
 // The two launches of an iteration with 16-byte vectors, face rows on sf.
 cudaError_t launch_rows(const lbm_t *h, int mode, const lbm::StepArgs &a, cudaStream_t sf)
 {
-    return h->prec == LBM_FP16 ? lbm::launch_rows_f16(mode, a, h->step_block, h->stream, sf)
-                               : lbm::launch_rows_bf16(mode, a, h->step_block, h->stream, sf);
+    switch (h->prec) {
+    case LBM_FP32: return lbm::launch_rows_f32(mode, a, h->step_block, h->stream, sf);
+    case LBM_FP16: return lbm::launch_rows_f16(mode, a, h->step_block, h->stream, sf);
+    default: return lbm::launch_rows_bf16(mode, a, h->step_block, h->stream, sf);
+    }
 }
 
 cudaError_t launch_pull(const lbm_t *h, int mode, const lbm::StepArgs &a, unsigned *nparts = nullptr)
@@ -341,8 +344,7 @@ cudaError_t launch_pull(const lbm_t *h, int mode, const lbm::StepArgs &a, unsign
     // them: 16-bit storage with 8-byte vectors at every size beyond 40^3 (us per
     // iteration of the adjoint forward, 16-byte vectors -> 8: FP16 96^3 15.1 ->
     // 14.5, 256^3 262 -> 250; BF16 128^3 38.6 -> 36.5, 256^3 278 -> 253).
-    const bool s16 = h->prec == LBM_FP16 || h->prec == LBM_BF16;
-    const int vb = mode == lbm::MODE_STEP_ADJ && s16 && h->step_vb != 4 ? 8 : h->step_vb;
+    const int vb = mode == lbm::MODE_STEP_ADJ && h->prec != LBM_FP64 && h->step_vb != 4 ? 8 : h->step_vb;
     if (!vb) return launch_rows(h, mode, a, h->stream);
     switch (h->prec) {
     case LBM_FP32: return lbm::launch_step_f32(vb, mode, a, h->step_block, h->stream);

@@ -91,11 +91,12 @@ cudaError_t LBM_CAT(launch_reduce_, LBM_SFX)(const StepArgs &a, unsigned block, 
     return launch_rows_mode<MODE_REDUCE>(a, block, s, nullptr, nparts);
 }
 
-// 16-bit storage only (large lattices; see step_shape in lbm_capi.cu).
+// (16-bit storage on large lattices, FP32 with 16-byte vectors; see step_shape
+// in lbm_capi.cu)
 cudaError_t LBM_CAT(launch_rows_, LBM_SFX)(int mode, const StepArgs &a, unsigned block, cudaStream_t s,
                                            cudaStream_t sf)
 {
-    if constexpr (sizeof(LBM_S) == 2) {
+    if constexpr (sizeof(LBM_S) < 8) {
         switch (mode) {
         case MODE_STEP: return launch_rows_mode<MODE_STEP>(a, block, s, sf, nullptr);
         case MODE_STEP_MACRO: return launch_rows_mode<MODE_STEP_MACRO>(a, block, s, sf, nullptr);
@@ -143,7 +144,9 @@ template <int VB> static cudaError_t launch_step_vb(int mode, const StepArgs &a,
 cudaError_t LBM_CAT(launch_step_, LBM_SFX)(int vb, int mode, const StepArgs &a, unsigned block, cudaStream_t s)
 {
     switch (vb) {
-    case 16: return launch_step_vb<16>(mode, a, block, s);
+    case 16:
+        if constexpr (sizeof(LBM_S) != 4) return launch_step_vb<16>(mode, a, block, s);
+        break;
     case 8: return launch_step_vb<8>(mode, a, block, s);
     case 4:
         if constexpr (sizeof(LBM_S) < 8) return launch_step_vb<4>(mode, a, block, s);
