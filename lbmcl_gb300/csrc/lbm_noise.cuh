@@ -8,10 +8,11 @@
 // feeds sample pairs 2g and 2g+1; populations 2m and 2m+1 of a site take
 // pair m.  The logarithm is summed from the atanh series, sine and cosine
 // from their Taylor series on a quarter turn (Horner steps as fused
-// multiply-adds).  Every floating-point step is an explicit IEEE
-// single-precision operation or fma (no contraction left to the compiler, no
-// library transcendental), so a CPU implementation of the same recipe gets
-// the same bits.  Single precision because FP64 runs at a small fraction of the FP32
+// multiply-adds).  Every floating-point step is an explicit single-precision
+// operation or fma with the IEEE result (no contraction left to the compiler, no
+// library transcendental; the division and the square root start from
+// approximations and are corrected with exact remainders), so a CPU
+// implementation of the same recipe gets the same bits.  Single precision because FP64 runs at a small fraction of the FP32
 // rate on GB300 and the samples only perturb the initial state.
 #pragma once
 
