@@ -194,7 +194,6 @@ lbm::StepArgs step_args(const lbm_t *h, int from, int phase)
     a.partials = h->partials;
     a.dim = h->dim;
     a.nvx = h->dim / h->V;
-    a.nvec = h->nvec;
     a.n = h->n;
     a.inv_tau = h->inv_tau;
     a.omega_f = h->omega_f;
@@ -645,8 +644,6 @@ int lbm_init(lbm_t **out, const lbm_config *c)
     h->V = V;
     h->sd = sd;
     h->block = block;
-    h->nvec = (unsigned)nvec;
-    h->grid = (unsigned)grid;
     h->base_bytes = need;
 
     // tau = 3 nu + 0.5 and 1/tau in the compute precision (kernels.cl:61-62)
@@ -735,7 +732,7 @@ int lbm_init(lbm_t **out, const lbm_config *c)
         // 32 threads 1539, 64 1527, 96 1556, 128 1558; FP32 200^3: 64 174.6,
         // 128 175.9, 256 183)
         h->step_block = c->block_threads > 0 ? block : 64u;
-        if (!h->step_vb) {
+        if (!h->step_vb && !aa && want != LBM_KERNEL_STAGED) {  // splits(h)
             LBM_CUDA(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
             LBM_CUDA(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
             LBM_CUDA(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));

@@ -391,7 +391,6 @@ struct StepArgs {
     double *partials;    // reduction partials, 2 per block
     int dim;
     int nvx;             // x-vectors per row = dim / V
-    unsigned nvec;       // vectors in the interior rows = nvx * (dim-2)^2
     unsigned partial_base;  // first reduction-partial slot of this launch
     size_t n;            // dim^3
     double inv_tau;      // 1/tau in the compute precision (rounded by the host)

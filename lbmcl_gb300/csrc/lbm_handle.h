@@ -84,8 +84,6 @@ struct lbm_handle {
     double kernels_ms = 0;
     int64_t it = 0;
     unsigned block = 128;
-    unsigned nvec = 0;
-    unsigned grid = 0;
     // staged variant (LBM_KERNEL_STAGED)
     int kernel = LBM_KERNEL_DIRECT;
     int step_vb = 16;         // vector bytes of the one-launch iteration; 0: two launches (step_shape)

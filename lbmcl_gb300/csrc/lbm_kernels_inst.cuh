@@ -36,7 +36,7 @@ static cudaError_t launch_rows_mode(const StepArgs &a0, unsigned block, cudaStre
 }
 
 // One AA iteration (or reduction pass) of phase PHASE: interior rows, then
-// face rows, as launch_direct.
+// face rows.
 template <int VB, int PHASE>
 static cudaError_t launch_aa_phase(int mode, const StepArgs &a0, unsigned block, cudaStream_t s, unsigned *nparts)
 {
@@ -136,7 +136,9 @@ template <int VB> static cudaError_t launch_step_vb(int mode, const StepArgs &a,
     switch (mode) {
     case MODE_STEP: return launch_step_mode<VB, MODE_STEP>(a, block, s);
     case MODE_STEP_MACRO: return launch_step_mode<VB, MODE_STEP_MACRO>(a, block, s);
-    case MODE_STEP_ADJ: return launch_step_mode<VB, MODE_STEP_ADJ>(a, block, s);
+    case MODE_STEP_ADJ:  // (16-bit storage: 8-byte vectors, launch_pull)
+        if constexpr (sizeof(LBM_S) != 2 || VB < 16) return launch_step_mode<VB, MODE_STEP_ADJ>(a, block, s);
+        return cudaErrorInvalidValue;
     default: return cudaErrorInvalidValue;
     }
 }
