@@ -271,7 +271,8 @@ int setup_staged(lbm_t *h, int want_stages)
 
 // Vector width and launch count of an iteration of the direct and narrow
 // variants: h->step_vb > 0, step_kernel with vectors of so many bytes, one
-// launch; 0, pull_kernel's two launches with 16-byte vectors (16-bit storage).
+// launch; 0, pull_kernel's two launches with 16-byte vectors (large 16-bit
+// lattices; FP32 DIRECT).
 //
 // Wide vectors cost registers and give few threads: a small lattice wants
 // one or two sites per thread (its time is the latency of one thread's work
@@ -279,18 +280,24 @@ int setup_staged(lbm_t *h, int want_stages)
 // replayed graphs, 4- / 8- / 16-byte vectors, one launch; two launches:
 //   FP16  32^3  2.4 / 2.4 / 4.1; 4.9   64^3 5.6 / 5.0 / 6.7; 6.0
 //         96^3 14.0 / 10.9 / 11.8; 12.4   112^3 - / 19.6 / 18.8
-//         128^3 34 / 28.9 / 29.0; 30.0   160^3 - / 54.4 / 55.0; 56.3
-//         200^3 - / 104.7 / 104.7; 103.3   256^3 - / 199 / 208; 203
-//         320^3 - / 398 / -; 389   512^3 - / 1604 / 1610; 1527
+//         128^3 34 / 29.4 / 29.3; 30.0   160^3 - / 55.0 / 55.5; 56.3
+//         200^3 - / 105.0 / 104.7; 103.7   256^3 - / 200 / 208; 205
+//         288^3 - / 299 / -; 292   320^3 - / 398 / -; 390   512^3 - / 1594 / 1610; 1527
 //   BF16  32^3  2.4 / 2.4 / 3.6; 6.0   64^3 5.6 / 5.0 / 6.5; 7.0
 //         96^3 13 / 11.4 / 11.6; 13.8   112^3 - / 19.8 / 18.5
-//         128^3 31.6 / 29.2 / 28.8; 31.4   200^3 - / 105.8 / 105.5; 106.2
-//         256^3 - / 201 / 208; 206   512^3 - / 1619 / 1597; 1560
+//         128^3 31.6 / 29.7 / 29.1; 31.4   200^3 - / 106.1 / 105.5; 106.5
+//         256^3 - / 202 / 208; 208   288^3 - / 302 / -; 297   320^3 - / 402 / -; 394
+//         512^3 - / 1608 / 1597; 1558
 //   FP32  32^3  2.9 / 3.2 / 4.9; 3.8   64^3 8.1 / 7.5 / 9.0; 7.9
 //         128^3 57 / 48.0 / 55; 50.7   256^3 400 / 360 / 415; 375
 //         512^3 3157 / 2910 / 3217; 2950
-//   FP64 (8- / 16-byte) 16^3 13.3 / 20.9; 24   32^3 19.6 / 23.9; 24
-//         128^3 989 / 1050; 1045   256^3 7767 / 8014; 7987
+//   FP64 (8- / 16-byte) 16^3 10.8 / 21.1   32^3 12.0 / 24.1   64^3 63 / 134
+//         128^3 467 / 1049   256^3 3480 / 8539
+// The 16-bit line at 192^3: two launches are 2 to 4% ahead from 288^3 up; between
+// it and 256^3 neither side is by more than 1.3%, but at 256^3 itself 8-byte
+// vectors in one launch are by 2.3% (FP16) and 2.8% (BF16): a line for that one size
+// would lose as much at 288^3.  FP32 DIRECT, the 16-byte vectors asked for: two
+// launches 56^3 7.6, 256^3 380 against 8.4 and 397 in one.
 int step_shape(int kernel, int prec, int dim)
 {
     const bool s16 = prec == LBM_FP16 || prec == LBM_BF16;
@@ -339,10 +346,12 @@ cudaError_t launch_pull(const lbm_t *h, int mode, const lbm::StepArgs &a, unsign
         default: return lbm::launch_staged_bf16(mode, a, h->sgrid, h->sblock, h->ssmem, h->stream);
         }
     }
-    // Iterations that also store the linearisation points need registers for
-    // them: 16-bit storage with 8-byte vectors at every size beyond 40^3 (us per
-    // iteration of the adjoint forward, 16-byte vectors -> 8: FP16 96^3 15.1 ->
-    // 14.5, 256^3 262 -> 250; BF16 128^3 38.6 -> 36.5, 256^3 278 -> 253).
+    // Iterations that also store the linearisation points: 8-byte vectors at
+    // every 16-bit size beyond 40^3 (us per iteration of the adjoint forward,
+    // 16-byte vectors -> 8: FP16 96^3 15.1 -> 14.5, 256^3 262 -> 250; BF16 128^3 38.6
+    // -> 36.5, 256^3 278 -> 253).  Not for spills: the FP16 kernel had none with
+    // 16-byte vectors and has 56 bytes at 128 registers with 8-byte ones, but
+    // 16 warps per SM instead of 12.
     const int vb = mode == lbm::MODE_STEP_ADJ && h->prec != LBM_FP64 && h->step_vb != 4 ? 8 : h->step_vb;
     if (!vb) return launch_rows(h, mode, a, h->stream);
     switch (h->prec) {

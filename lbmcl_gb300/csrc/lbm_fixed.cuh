@@ -7,10 +7,11 @@
 // cycle beside it; the update is 260 FP64 operations a site in IEEE operations,
 // 80 here, and 4,500 integer instructions.  256^3: 7767 -> 3470 us per
 // iteration (2110 -> 4722 MLUPS, 9% -> 21% of HBM), 64^3 133 -> 62.9, 32^3 19.6 ->
-// 12.0 (ncu at 128^3: FP64 pipe 64% active, integer pipe 60%).  The last sum of
-// every population on the FP64 pipe too (19 operations more, a seventh of the
-// integer instructions less): 256^3 4436.  At 128 registers, 16 warps per SM
-// (254 registers, 8 warps: 4698; 80 registers with spills: 3779).
+// 12.0 (ncu at 256^3: FP64 pipe 61% active, integer pipe 70%).  Left out, against
+// 3777 before the warps left the windows together: the last sum of every
+// population on the FP64 pipe too (19 operations more, a seventh of the integer
+// instructions less) 4436; 254 registers, 8 warps per SM instead of 16, 4698; 80
+// registers with spills 3779.
 //
 // Between values whose binary exponents are known to lie in a small
 // window, an IEEE addition is an integer addition and one rounding to 53

@@ -2,7 +2,7 @@
 //
 //   step_kernel<S, MODE>  one fused pull-stream + collide iteration
 //                         (replaces kernels.cl:321-425)
-//   pull_kernel<S, MODE>  the same in two launches (large 16-bit lattices);
+//   pull_kernel<S, MODE>  the same in two launches (step_shape says where);
 //                         MODE_REDUCE reuses its gather to form FP64 mass /
 //                         energy partials
 //   init_kernel<S>        initial state (replaces kernels.cl:277-318)
@@ -607,8 +607,8 @@ __device__ __forceinline__ void update_general(S (&fs)[Q][V], typename MapWord<V
 // bits either way): 0 = two scalar site updates, 2 = packed FP32x2.  Packed is
 // a fifth fewer instructions; FP16 with eight sites per thread spills 80 bytes
 // that way at the 168-register cap and is scalar there (512^3 84,999 MLUPS
-// against 81,241; with four sites per thread, no spills, packed: 96^3 12.0 ->
-// 10.9 us, 256^3 211 -> 200).
+// against 81,241); with four sites per thread it spills 8 bytes at 128 registers
+// and is packed (96^3 12.0 -> 10.9 us, 256^3 211 -> 200).
 template <class S, int V> __host__ __device__ constexpr int dev16_form()
 {
     return sizeof(S) != 2 || (std::is_same<S, __half>::value && V == 8) ? 0 : 2;

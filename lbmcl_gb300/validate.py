@@ -225,20 +225,19 @@ def lidfield(args):
         fwd_ms = e0.elapsed_time(e1) / 100
 
     def run_adjoint(prec, every, a64=False):
-        capi.keep_memory(0)  # what earlier handles left idle is not this run's
-        capi.keep_memory()
-        free0, _ = torch.cuda.mem_get_info()
         with capi.Lattice(dim, velocity=0.0, precision=prec, lid=lid, tau=tau, stride=0, adjoint_fp64=a64) as L:
             L.adjoint_set_loss(plane, target)
             torch.cuda.synchronize()
             t0 = time.perf_counter()
             J = L.adjoint_forward(steps, every)
             t1 = time.perf_counter()
-            free1, _ = torch.cuda.mem_get_info()
             _, gl, _ = L.adjoint_backward(1.0, want_f0=False, want_tau=False)
             t2 = time.perf_counter()
-            free2, _ = torch.cuda.mem_get_info()
-        return J, gl, t1 - t0, t2 - t1, (free0 - min(free1, free2)) / 1e9
+            capi.keep_memory(0)  # the handle holds all that the two took; what others left idle goes
+            inside, _ = torch.cuda.mem_get_info()
+        after, _ = torch.cuda.mem_get_info()
+        capi.keep_memory()
+        return J, gl, t1 - t0, t2 - t1, (after - inside) / 1e9
 
     J, g32, tf, tb, gb = run_adjoint(args.precision, c)
     out.update({"loss": J, "forward_ms_per_iter": round(fwd_ms, 4),

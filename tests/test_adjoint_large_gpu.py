@@ -51,3 +51,23 @@ def test_large_gradient(capi, prec, tau, how):
         for a, b in zip(base[2:4], wide[2:4]):
             a, b = a.astype(np.float64), b.astype(np.float64)
             assert np.linalg.norm(a - b) <= 3 * T * 2.0 ** -24 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("tau", [False, True])
+@pytest.mark.parametrize("graphs", [0, 1])
+def test_direct_fp32_gradient(capi, tau, graphs):
+    """FP32 DIRECT iterations are two forked launches at every size; their points
+    come from the one-launch kernel: the gradient of the default variant."""
+    dim, got = 40, []
+    lid = 0.05 + 0.005 * np.random.default_rng(4).standard_normal(dim * dim)
+    for kernel in (0, "direct"):
+        for tail in (-1, 0):
+            with capi.Lattice(dim, velocity=0.0, precision="fp32", lid=lid, tau=0.53, seed=3, noise_sigma=1e-4,
+                              kernel=kernel, graph_iterations=graphs, adjoint_tail_segments=tail) as L:
+                L.adjoint_set_loss(dim // 2, None)
+                J = L.adjoint_forward(23, 6)
+                got.append((J,) + L.adjoint_backward(1.0, want_tau=tau) + (L.f(),))
+    for other in got[1:]:
+        assert got[0][0] == other[0] and got[0][1] == other[1]
+        for a, b in zip(got[0][2:], other[2:]):
+            np.testing.assert_array_equal(a, b)
